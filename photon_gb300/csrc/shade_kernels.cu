@@ -24,25 +24,29 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
   // step or a density lookup), ending at its next lookup
   const uint32_t n = wc.count[it];
   uint32_t *fetch = wc.vfetch + 2 * it;
+  const uint32_t per_warp = spread_lanes(n);
+  // lanes of this warp that take rays
+  const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
+  const uint32_t refill_at = min(wc.vol_refill, (per_warp + 1u) >> 1);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   VolTrack s;
   Rng rng(1u);
   bool busy = false, exhausted = false;
-  uint32_t idx = 0, idle = WARP_FULL, nlook = 0;
+  uint32_t idx = 0, idle = lanes_on, nlook = 0;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) { // warp-uniform
       if (lane == 0)
         atomicCAS(wc.error, 0u, (WAVE_ERR_VOLUME << 16) | uint32_t(it));
       break;
     }
-    if (!exhausted && (idle == WARP_FULL || uint32_t(__popc(idle)) >= wc.vol_refill)) {
+    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
       const uint32_t k = uint32_t(__popc(idle));
       const uint32_t base = warp_fetch(fetch, k);
       if (base + k >= n)
         exhausted = true;
-      if (!busy) {
+      if ((idle >> lane) & 1u) {
         const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
         if (my < n) {
           idx = my;
@@ -54,9 +58,9 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
           busy = true;
         }
       }
-      idle = __ballot_sync(WARP_FULL, !busy);
+      idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
-    if (idle == WARP_FULL) {
+    if (idle == lanes_on) {
       if (exhausted)
         break;
       continue;
@@ -70,7 +74,7 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
       }
     }
     __syncwarp(); // every lane back from the step's divergent work before the vote
-    idle = __ballot_sync(WARP_FULL, !busy);
+    idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
   }
   if (lookups) { // the loop ends for the whole warp at once
     const uint32_t w = __reduce_add_sync(WARP_FULL, nlook);

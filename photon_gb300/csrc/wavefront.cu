@@ -214,6 +214,10 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
     return;
   const uint32_t n = wc.count[it];
   uint32_t *fetch = wc.fetch + 4 * it;
+  const uint32_t per_warp = spread_lanes(n);
+  // lanes of this warp that take rays
+  const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
+  const uint32_t refill_at = min(refill, (per_warp + 1u) >> 1);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   TravCounters ctr{0u, 0u};
@@ -225,21 +229,21 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
   const float4 *tris = sc.tris;
   // The idle mask changes only when lanes finish or fetch, so the warp votes
   // (refill, queue appends) run only on trips where some lane finished.
-  uint32_t idle = WARP_FULL;
+  uint32_t idle = lanes_on;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) { // warp-uniform: every lane counts the same trips
       record_cap(wc, (WAVE_ERR_TRACE << 16) | uint32_t(it), n, *fetch, busy, exhausted, idx, in.ray_o[idx],
           in.ray_d[idx], s, steps, rays, fetch_trips, step_trips, max_steps, max_idx, trips);
       break;
     }
-    if (!exhausted && (idle == WARP_FULL || uint32_t(__popc(idle)) >= refill)) {
+    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
       const uint32_t k = uint32_t(__popc(idle));
       const uint32_t base = warp_fetch(fetch, k);
       ++fetch_trips;
       if (base + k >= n)
         exhausted = true;
-      if (!busy) {
+      if ((idle >> lane) & 1u) {
         const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
         if (my < n) {
           idx = my;
@@ -258,9 +262,9 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
           busy = true;
         }
       }
-      idle = __ballot_sync(WARP_FULL, !busy);
+      idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
-    if (idle == WARP_FULL) {
+    if (idle == lanes_on) {
       if (exhausted)
         break;
       continue;
@@ -444,6 +448,10 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
     return;
   const uint32_t n = wc.scount[it];
   uint32_t *fetch = wc.fetch + 4 * it + 3;
+  const uint32_t per_warp = spread_lanes(n);
+  // lanes of this warp that take rays
+  const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
+  const uint32_t refill_at = min(refill, (per_warp + 1u) >> 1);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   TravCounters ctr{0u, 0u};
@@ -455,21 +463,21 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
   const float4 *tris = sc.tris;
   // persistent warps with dynamic refill, as in k_trace: the idle mask
   // changes only where lanes finish or fetch
-  uint32_t idle = WARP_FULL;
+  uint32_t idle = lanes_on;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) {
       record_cap(wc, (WAVE_ERR_SHADOW << 16) | uint32_t(it), n, *fetch, busy, exhausted, idx, sh.a[idx], sh.b[idx],
           s, steps, rays, fetch_trips, step_trips, max_steps, max_idx, trips);
       break;
     }
-    if (!exhausted && (idle == WARP_FULL || uint32_t(__popc(idle)) >= refill)) {
+    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
       const uint32_t k = uint32_t(__popc(idle));
       const uint32_t base = warp_fetch(fetch, k);
       ++fetch_trips;
       if (base + k >= n)
         exhausted = true;
-      if (!busy) {
+      if ((idle >> lane) & 1u) {
         const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
         if (my < n) {
           idx = my;
@@ -488,9 +496,9 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
           busy = true;
         }
       }
-      idle = __ballot_sync(WARP_FULL, !busy);
+      idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
-    if (idle == WARP_FULL) {
+    if (idle == lanes_on) {
       if (exhausted)
         break;
       continue;
@@ -534,7 +542,7 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
         sh.a[idx].w = -1.f;
     }
     __syncwarp(); // every lane back from the step's divergent work before the vote
-    idle = __ballot_sync(WARP_FULL, !busy);
+    idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
   }
   if (COUNT) {
     atomicAdd((unsigned long long *)&stats[0], (unsigned long long)ctr.nodes);
@@ -558,25 +566,29 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
   // one tracking pass per busy lane and trip, as in k_vol_scatter
   const uint32_t n = wc.scount[it];
   uint32_t *fetch = wc.vfetch + 2 * it + 1;
+  const uint32_t per_warp = spread_lanes(n);
+  // lanes of this warp that take rays
+  const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
+  const uint32_t refill_at = min(wc.vol_refill, (per_warp + 1u) >> 1);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   VolTrack s;
   Rng rng(1u);
   bool busy = false, exhausted = false;
-  uint32_t idx = 0, job = 0, idle = WARP_FULL, nlook = 0;
+  uint32_t idx = 0, job = 0, idle = lanes_on, nlook = 0;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) { // warp-uniform
       if (lane == 0)
         atomicCAS(wc.error, 0u, (WAVE_ERR_VOLUME << 16) | uint32_t(it));
       break;
     }
-    if (!exhausted && (idle == WARP_FULL || uint32_t(__popc(idle)) >= wc.vol_refill)) {
+    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
       const uint32_t k = uint32_t(__popc(idle));
       const uint32_t base = warp_fetch(fetch, k);
       if (base + k >= n)
         exhausted = true;
-      if (!busy) {
+      if ((idle >> lane) & 1u) {
         const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
         if (my < n) {
           const float4 a = sh.a[my];
@@ -591,9 +603,9 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
           }
         }
       }
-      idle = __ballot_sync(WARP_FULL, !busy);
+      idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
-    if (idle == WARP_FULL) {
+    if (idle == lanes_on) {
       if (exhausted)
         break;
       continue;
@@ -617,7 +629,7 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
       }
     }
     __syncwarp(); // every lane back from the step's divergent work before the vote
-    idle = __ballot_sync(WARP_FULL, !busy);
+    idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
   }
   if (lookups) { // the loop ends for the whole warp at once
     const uint32_t w = __reduce_add_sync(WARP_FULL, nlook);
