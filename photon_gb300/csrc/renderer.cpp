@@ -104,6 +104,8 @@ struct phc_renderer {
   Buf sort_bins; // per bounce iteration: material-sort counts and starts
   size_t cap_slots{0};
   Buf acc, acc_sq, acc_start, nsamp, aov_n, aov_a;
+  Buf ad_pixels, ad_planes; // adaptive sampling with several samples in flight (AdaptState)
+  size_t ad_clear{0};       // bytes of ad_planes known to be zero
   Buf counters; // count, scount, fetch, wave, error
   Buf rc_buf, stats_buf, bg_buf;
   size_t bg_floats{0};
@@ -236,6 +238,7 @@ void check_device(phc_renderer *r) { ck(cudaSetDevice(r->device), "cudaSetDevice
 void ensure_path_state(phc_renderer *r, size_t n)
 {
   r->buf_gen++;
+  r->cap_paths = 0; // until every buffer is there: a failed growth leaves none behind
   for (int b = 0; b < 2; ++b) {
     ck(r->st_o[b].ensure(n * 16), "alloc path state");
     ck(r->st_d[b].ensure(n * 16), "alloc path state");
@@ -260,6 +263,7 @@ void ensure_paths(phc_renderer *r, size_t n)
     ensure_path_state(r, n);
   if (r->scene.dev.volume_count > 0 && r->cap_vol < r->cap_paths) {
     r->buf_gen++;
+    r->cap_vol = 0;
     ck(r->vol_scatter.ensure(r->cap_paths * 16), "alloc volume scattering");
     ck(r->vol_rng.ensure(r->cap_paths * 4), "alloc volume scattering");
     ck(r->vol_q.ensure(r->cap_paths * 4), "alloc volume scattering");
@@ -272,6 +276,7 @@ void ensure_slots(phc_renderer *r, size_t n)
   if (n <= r->cap_slots)
     return;
   r->buf_gen++;
+  r->cap_slots = 0;
   ck(r->acc.ensure(n * 16), "alloc accumulators");
   ck(r->acc_sq.ensure(n * 16), "alloc accumulators");
   ck(r->acc_start.ensure(n * 16), "alloc accumulators");
@@ -373,13 +378,15 @@ struct KernelTimer {
 // wave_paths: paths of one wave (lanes x pixels); the material sort and the
 // class kernels are recorded only where an iteration can reach the sort
 // threshold.
+// ad: the state of an adaptive wave with several samples in flight (planes
+// not null), whose contributions go to its planes instead of the accumulators.
 uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, const RenderConst *rc, uint32_t npix,
-    size_t wave_paths, int max_iter, int adaptive, bool counting, KernelTimer *tm = nullptr)
+    size_t wave_paths, int max_iter, int adaptive, bool counting, const AdaptState &ad, KernelTimer *tm = nullptr)
 {
   const WaveCounters wc = wave_counters(r, max_iter);
   ck(cudaMemsetAsync(wc.count, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
   const DevScene sc = r->scene.dev;
-  const Accum ac = accum(r);
+  const Accum acc_all = accum(r);
   const ShadowSoA sh{r->sh_a.as<float4>(), r->sh_b.as<float4>(), r->sh_c.as<float4>()};
   uint64_t *stats = r->stats_buf.as<uint64_t>();
   auto timed = [&](int kind, auto &&launch) {
@@ -434,10 +441,15 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
   uint64_t launches = 2;
   if (tm)
     tm->begin_wave();
-  timed(0, [&] { launch_raygen(cfg, s, rc, sc, path_soa(r, 0), ac, wc); });
+  timed(0, [&] { launch_raygen(cfg, s, rc, sc, path_soa(r, 0), acc_all, wc, ad); });
   for (int it = 0; it < max_iter; ++it) {
     const PathSoA in = path_soa(r, it & 1), out = path_soa(r, (it + 1) & 1);
     float4 *hits = r->hits.as<float4>();
+    Accum ac = acc_all, ac_shadow = acc_all;
+    if (ad.planes) {
+      ac.acc = ad.planes + size_t(2 * it) * wave_paths;
+      ac_shadow.acc = ac.acc + wave_paths;
+    }
     HitQueues hq_trace = hq;
     if (vsplit) // the tracking pre-pass writes the queues
       hq_trace.hitq = hq_trace.missq = nullptr;
@@ -480,13 +492,21 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
       timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 0}, hq); });
       launches += 3;
     }
-    timed(3, [&] { launch_shadow(cfg, s, rc, sc, sh, ac, wc, it, counting ? stats + 5 : nullptr, tu.trace_refill); });
+    timed(3, [&] { launch_shadow(cfg, s, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 5 : nullptr, tu.trace_refill); });
     if (sc.volume_count > 0) {
-      timed(6, [&] { launch_shadow_volume(cfg, s, rc, sc, sh, ac, wc, it, counting ? stats + 7 : nullptr); });
+      timed(6, [&] { launch_shadow_volume(cfg, s, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 7 : nullptr); });
       launches += 1;
     }
   }
-  timed(4, [&] { launch_wave_end(s, rc, ac, wc, npix, adaptive, max_iter, stats); });
+  if (ad.planes) {
+    timed(4, [&] {
+      launch_adapt_merge(s, rc, ad, acc_all, wc, npix, uint32_t(wave_paths), max_iter, stats);
+    });
+    launches += 1;
+  }
+  timed(4, [&] {
+    launch_wave_end(s, rc, acc_all, wc, npix, ad.planes ? 0 : adaptive, max_iter, stats, !ad.planes);
+  });
   if (tm)
     tm->end_wave(s);
   return launches;
@@ -521,6 +541,10 @@ void check_wave_error(uint32_t w, const WaveCounters &wc, cudaStream_t s)
           std::to_string(d[21]) + "); trips " + std::to_string(d[22]) + " active " + std::to_string(d[23]) + ")");
 }
 
+// adapt_lanes: paths of an adaptive wave and the bytes of its accumulator planes
+constexpr uint64_t ADAPT_PATHS = 1ull << 25;
+constexpr uint64_t ADAPT_PLANE_BYTES = 24ull << 30;
+
 // What one render call of one renderer needs: its constants, sample lanes
 // and wave count; prepared (buffers sized, accumulators zeroed) on stream s.
 struct JobPlan {
@@ -529,6 +553,7 @@ struct JobPlan {
   int max_iter{0};
   size_t slots{0};
   bool first{true};
+  AdaptState ad{}; // planes not null: adaptive sampling with several samples in flight
 };
 
 void validate_call(phc_renderer *r, const phc_settings &st)
@@ -578,6 +603,47 @@ RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg,
   return rc;
 }
 
+// Samples of one pixel that an adaptive wave traces side by side (AdaptState),
+// a power of two up to 16; 1: waves of one sample each.  One sample of a
+// 640 x 360 frame leaves most of the GPU waiting for the longest paths, and
+// even 3.7M paths (1920 x 1920) do.  Measured through the 2M-triangle volume
+// scene at 64 spp (Msamples/s; 1920 x 1920, 1920 x 1080, 1280 x 720): one
+// sample per wave 260 / 205 / 115; waves of up to 2^23 paths 342 / 402 / 386,
+// 2^24 411 / 488 / 477, 2^25 454 / 543 / 476.  A pixel whose gate closes in
+// mid-wave has up to 15 samples traced for nothing; over these frames that is
+// at most 1e-6 of the rays, since most closing pixels do so at the first gate.
+// Frames with no room for two samples keep one per wave.
+uint32_t adapt_lanes(const RenderConst &rc, uint64_t wave_paths)
+{
+  const uint64_t paths = std::min(ADAPT_PATHS, wave_paths);
+  uint32_t n = 1;
+  while (n < ADAPT_MIN_SAMPLES && n < rc.spp && uint64_t(2 * n) * rc.npix <= paths &&
+      uint64_t(2 * n) * rc.npix * 2 * rc.max_iter * 16 <= ADAPT_PLANE_BYTES)
+    n *= 2;
+  return n;
+}
+
+// Buffers of an adaptive call with `lanes` samples in flight; false when the
+// device has no room for them.
+bool ensure_adaptive(phc_renderer *r, uint32_t npix, uint32_t lanes, int max_iter)
+{
+  const size_t slots = size_t(lanes) * npix;
+  const size_t pixel_bytes = size_t(npix) * (5 * 16 + 4), plane_bytes = size_t(2) * max_iter * slots * 16;
+  if (r->ad_pixels.bytes >= pixel_bytes && r->ad_planes.bytes >= plane_bytes)
+    return true;
+  r->ad_clear = 0;
+  r->buf_gen++;
+  cudaError_t e = r->ad_pixels.ensure(pixel_bytes);
+  if (e == cudaSuccess)
+    e = r->ad_planes.ensure(plane_bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError(); // dealt with here
+    return false;
+  }
+  ck(e, "alloc adaptive state");
+  return true;
+}
+
 JobPlan prepare_job(phc_renderer *r, const phc_camera &cam, const phc_settings &st, bool reset, cudaStream_t s)
 {
   validate_call(r, st);
@@ -595,14 +661,17 @@ JobPlan prepare_job(phc_renderer *r, const phc_camera &cam, const phc_settings &
   }
   RenderConst rc = render_const(cam, st, r->bg_buf, s);
   rc.sample_offset = r->sample_counter;
-  // samples of one pixel in flight: enough paths to fill the GPU, one when
-  // adaptive sampling needs the samples in order
+  // samples of one pixel in flight: enough paths to fill the GPU
   const Tuning &tu = tuning();
   uint32_t lanes = 1;
   if (!rc.adaptive) {
     const uint64_t target = tu.wave_paths;
     lanes = uint32_t(std::min<uint64_t>(rc.spp, std::max<uint64_t>(1, (target + npix - 1) / npix)));
     lanes = std::min<uint32_t>(lanes, std::max<uint32_t>(1u, uint32_t((1ull << 28) / npix)));
+  } else {
+    lanes = adapt_lanes(rc, uint64_t(tu.wave_paths));
+    if (lanes > 1 && !ensure_adaptive(r, npix, lanes, int(rc.max_iter)))
+      lanes = 1; // no room for the planes: one sample per wave
   }
   rc.lanes = lanes;
   JobPlan p;
@@ -615,6 +684,19 @@ JobPlan prepare_job(phc_renderer *r, const phc_camera &cam, const phc_settings &
   ensure_slots(r, p.slots);
   ensure_wave_buffers(r, p.max_iter);
   ck(cudaMemcpyAsync(r->rc_buf.p, &rc, sizeof(rc), cudaMemcpyHostToDevice, s), "upload constants");
+  if (rc.adaptive && lanes > 1) {
+    const size_t plane_bytes = size_t(2) * p.max_iter * p.slots * 16;
+    float4 *px = r->ad_pixels.as<float4>();
+    p.ad = AdaptState{px, px + npix, px + 2 * size_t(npix), reinterpret_cast<uint32_t *>(px + 5 * size_t(npix)),
+        px + 3 * size_t(npix), px + 4 * size_t(npix), r->ad_planes.as<float4>()};
+    ck(cudaMemsetAsync(px, 0, size_t(npix) * (5 * 16 + 4), s), "reset adaptive state");
+    if (r->ad_clear < plane_bytes) // k_adapt_merge leaves the planes cleared
+      ck(cudaMemsetAsync(r->ad_planes.p, 0, r->ad_planes.bytes, s), "reset adaptive planes");
+    r->ad_clear = 0; // until the call has ended well
+    ck(cudaMemsetAsync(r->aov_a.p, 0, p.slots * 16, s), "reset accumulators");
+    p.rc = rc;
+    return p;
+  }
   ck(cudaMemsetAsync(r->acc.p, 0, p.slots * 16, s), "reset accumulators");
   ck(cudaMemsetAsync(r->nsamp.p, 0, p.slots * 4, s), "reset accumulators");
   ck(cudaMemsetAsync(r->aov_a.p, 0, p.slots * 16, s), "reset accumulators");
@@ -681,7 +763,7 @@ void render_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st,
   KernelTimer timer;
   if (tu.time_kernels) {
     for (uint32_t wv = 0; wv < waves; ++wv)
-      launches += record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting, &timer);
+      launches += record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting, plan.ad, &timer);
   } else if (tu.use_graph) {
     if (!r->graph || std::memcmp(key, r->graph_key, sizeof(key)) != 0) {
       if (r->graph) {
@@ -691,7 +773,7 @@ void render_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st,
       cudaGraph_t g = nullptr;
       ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
       try {
-        r->graph_launches = record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting);
+        r->graph_launches = record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting, plan.ad);
       } catch (...) {
         cudaStreamEndCapture(s, &g);
         if (g)
@@ -710,12 +792,15 @@ void render_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st,
     launches = uint64_t(waves) * r->graph_launches;
   } else {
     for (uint32_t wv = 0; wv < waves; ++wv)
-      launches += record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting);
+      launches += record_wave(r, s, cfg, drc, npix, plan.slots, max_iter, rc.adaptive, counting, plan.ad);
   }
   const Frame fr = frame_of(r);
   if (tu.time_kernels)
     timer.mark(s, 4);
-  launch_resolve(s, accum(r), fr, npix, lanes, float(rc.spp), first ? 1 : 0);
+  Accum sums = accum(r);
+  if (plan.ad.planes)
+    sums = Accum{plan.ad.acc, nullptr, nullptr, plan.ad.nsamp, plan.ad.aov_n, plan.ad.aov_a};
+  launch_resolve(s, sums, fr, npix, plan.ad.planes ? 1 : lanes, float(rc.spp), first ? 1 : 0);
   if (tu.time_kernels) {
     timer.done(s);
     ck(cudaStreamSynchronize(s), "resolve");
@@ -733,6 +818,8 @@ void render_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st,
   ck(cudaMemcpyAsync(&err_word, wc.error, 4, cudaMemcpyDeviceToHost, s), "read error word");
   ck(cudaStreamSynchronize(s), "render");
   check_wave_error(err_word, wc, s);
+  if (plan.ad.planes)
+    r->ad_clear = r->ad_planes.bytes;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, r->ev0, r->ev1);
   r->last.pixel_samples = stats[0];
@@ -1108,7 +1195,7 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
     ck(cudaMemsetAsync(r->nsamp.p, 0, size_t(cnt) * npix * 4, s), "reset accumulators");
     ck(cudaMemsetAsync(r->aov_a.p, 0, size_t(cnt) * npix * 16, s), "reset accumulators");
     ck(cudaMemsetAsync(wc.wave, 0, 8, s), "reset wave");
-    record_wave(r, s, cfg, drc, npix, size_t(cnt) * npix, max_iter, 0, false);
+    record_wave(r, s, cfg, drc, npix, size_t(cnt) * npix, max_iter, 0, false, AdaptState{});
     // pass 2: the replay, bounce by bounce
     ck(cudaMemsetAsync(wc.count, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
     ck(cudaMemsetAsync(wc.wave, 0, 4, s), "reset wave");

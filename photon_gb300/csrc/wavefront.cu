@@ -70,19 +70,59 @@ __global__ void __launch_bounds__(256) k_raygen_batch(BatchTable bt, PathSoA out
   }
 }
 
+// The variance gate of adaptive sampling (pathtracer.cpp:710-725): whether a
+// pixel with sums a, squared values q and ns samples takes sample s.
+__device__ __forceinline__ bool adapt_open(float4 a, float4 q, uint32_t ns, uint32_t s)
+{
+  if (s < ADAPT_MIN_SAMPLES || ns < ADAPT_MIN_SAMPLES)
+    return true;
+  const V3 mean = V3{a.x, a.y, a.z} * (1.f / float(ns));
+  const V3 sq = V3{q.x, q.y, q.z} * (1.f / float(ns));
+  const V3 var = sq - V3{mean.x * mean.x, mean.y * mean.y, mean.z * mean.z};
+  const float max_var = fmaxf(var.x, fmaxf(var.y, var.z));
+  const float l = fmaxf(0.2126f * mean.x + 0.7152f * mean.y + 0.0722f * mean.z, 1e-4f);
+  return !(max_var / (l * l) < 0.01f);
+}
+
+// pt_update_variance (pathtracer.cpp:1129-1139): the squared difference of the
+// sums since the pixel's last sample began.  The reference adds it after
+// every sample of the frame, also for a pixel that did not take it.
+__device__ __forceinline__ float4 adapt_square(float4 q, float4 a, float4 start)
+{
+  const V3 sv = V3{a.x, a.y, a.z} - V3{start.x, start.y, start.z};
+  q.x = q.x + sv.x * sv.x;
+  q.y = q.y + sv.y * sv.y;
+  q.z = q.z + sv.z * sv.z;
+  return q;
+}
+
+// The first sample of the wave (0 .. cnt) that pixel p takes; a refused one
+// only adds its last sample's square again (q is brought up to that sample).
+// Every sample from there on is traced: whether the pixel takes the later
+// ones is known once their predecessors are.
+__device__ __forceinline__ uint32_t adapt_first(const AdaptState &ad, uint32_t p, uint32_t s0, uint32_t cnt,
+    float4 a, float4 start, uint32_t ns, float4 &q)
+{
+  uint32_t l = 0;
+  for (; l < cnt && !adapt_open(a, q, ns, s0 + l); ++l)
+    q = adapt_square(q, a, start);
+  return l;
+}
+
 __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ rcp, DevScene sc, PathSoA out,
-    Accum acc, WaveCounters wc)
+    Accum acc, WaveCounters wc, AdaptState ad)
 {
   const RenderConst &rc = *rcp;
   const uint32_t wave = *wc.wave;
-  const uint32_t total = rc.npix * rc.lanes;
   // Without adaptive sampling the live slots are a prefix of the slot order
   // (lane-major: the lanes below spp - wave * lanes), so the queue is the slot
   // order itself: position = slot, no atomic per warp.
   const bool dense = !rc.adaptive;
+  const bool side_by_side = rc.adaptive && rc.lanes > 1u;
+  const uint32_t s0 = wave * rc.lanes;
+  const uint32_t total = rc.npix * rc.lanes;
   if (dense) {
-    const uint32_t first = wave * rc.lanes;
-    const uint32_t live_lanes = first < rc.spp ? min(rc.lanes, rc.spp - first) : 0u;
+    const uint32_t live_lanes = s0 < rc.spp ? min(rc.lanes, rc.spp - s0) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
       wc.count[0] = live_lanes * rc.npix;
   }
@@ -97,28 +137,25 @@ __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ 
       const uint32_t lane = i / rc.npix;
       pixel = i - lane * rc.npix;
       slot = i;
-      const uint32_t s = wave * rc.lanes + lane; // sample number within the render call
+      const uint32_t s = s0 + lane; // sample number within the render call
       if (s < rc.spp) {
         live = true;
-        if (rc.adaptive && s >= 16u) { // variance gate (pathtracer.cpp:710-725), lanes == 1
-          const uint32_t ns = acc.nsamp[slot];
-          if (ns >= 16u) {
-            const float4 a = acc.acc[slot], q = acc.acc_sq[slot];
-            const V3 mean = V3{a.x, a.y, a.z} * (1.f / float(ns));
-            const V3 sq = V3{q.x, q.y, q.z} * (1.f / float(ns));
-            const V3 var = sq - V3{mean.x * mean.x, mean.y * mean.y, mean.z * mean.z};
-            const float max_var = fmaxf(var.x, fmaxf(var.y, var.z));
-            const float l = fmaxf(0.2126f * mean.x + 0.7152f * mean.y + 0.0722f * mean.z, 1e-4f);
-            if (max_var / (l * l) < 0.01f)
-              live = false;
+        if (rc.adaptive && s >= ADAPT_MIN_SAMPLES) {
+          if (side_by_side) {
+            float4 q = ad.sq[pixel];
+            live = lane >= adapt_first(ad, pixel, s0, lane + 1u, ad.acc[pixel], ad.start[pixel], ad.nsamp[pixel], q);
+          } else { // lanes == 1
+            live = adapt_open(acc.acc[slot], acc.acc_sq[slot], acc.nsamp[slot], s);
           }
         }
         if (live) {
           sample_index = s + rc.sample_offset;
           camera_ray(rc, pixel, sample_index, ro, rd, tmin, tmax);
-          if (rc.adaptive)
-            acc.start[slot] = acc.acc[slot];
-          acc.nsamp[slot] += 1u;
+          if (!side_by_side) {
+            if (rc.adaptive)
+              acc.start[slot] = acc.acc[slot];
+            acc.nsamp[slot] += 1u;
+          }
         }
       }
     }
@@ -131,6 +168,83 @@ __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ 
       out.pdist[o] = 0.f;
     }
   }
+}
+
+// One thread per pixel: the wave's samples in order, each behind the gate,
+// its contributions bounce by bounce.  Iterations no path reached are skipped
+// (their planes are untouched); what is read is cleared for the next wave,
+// also of samples that turn out to be refused.  Bound by HBM (16 B per slot
+// and touched plane).
+__global__ void __launch_bounds__(256) k_adapt_merge(const RenderConst *__restrict__ rcp, AdaptState ad, Accum lanes,
+    WaveCounters wc, uint32_t npix, uint32_t slots, int max_iter, unsigned long long *accepted)
+{
+  if (wave_failed(wc))
+    return;
+  const RenderConst &rc = *rcp;
+  const uint32_t s0 = *wc.wave * rc.lanes;
+  const uint32_t cnt = s0 < rc.spp ? min(rc.lanes, rc.spp - s0) : 0u;
+  int iters = 0; // iterations that had paths (or shadow rays, which come from paths)
+  while (iters < max_iter && wc.count[iters] != 0u)
+    ++iters;
+  uint32_t taken = 0;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+    float4 a = ad.acc[p], q = ad.sq[p], start = ad.start[p];
+    uint32_t ns = ad.nsamp[p];
+    float4 aa = ad.aov_a[p];
+    uint32_t l = adapt_first(ad, p, s0, cnt, a, start, ns, q);
+    for (; l < cnt; ++l) {
+      const size_t slot = size_t(l) * npix + p;
+      const bool open = adapt_open(a, q, ns, s0 + l);
+      if (open) {
+        start = a;
+        ++ns;
+        ++taken;
+      }
+      for (int it = 0; it < iters; ++it) {
+        float4 *sp = ad.planes + size_t(2 * it) * slots + slot;
+        const float4 c = *sp;
+        if (!(c.x == 0.f && c.y == 0.f && c.z == 0.f && c.w == 0.f)) {
+          *sp = zero;
+          if (open) {
+            a.x = a.x + c.x;
+            a.y = a.y + c.y;
+            a.z = a.z + c.z;
+            a.w = a.w + c.w;
+          }
+        }
+        if (wc.scount[it] != 0u) {
+          float4 *np = sp + slots;
+          const float4 n = *np;
+          if (!(n.x == 0.f && n.y == 0.f && n.z == 0.f)) {
+            *np = zero;
+            if (open) {
+              a.x = a.x + n.x;
+              a.y = a.y + n.y;
+              a.z = a.z + n.z;
+            }
+          }
+        }
+      }
+      const float4 la = lanes.aov_a[slot];
+      if (__float_as_uint(la.w) != 0u) {
+        lanes.aov_a[slot] = zero;
+        if (open && __float_as_uint(aa.w) == 0u) {
+          aa = la;
+          ad.aov_a[p] = aa;
+          ad.aov_n[p] = lanes.aov_n[slot];
+        }
+      }
+      q = adapt_square(q, a, start);
+    }
+    ad.acc[p] = a;
+    ad.sq[p] = q;
+    ad.start[p] = start;
+    ad.nsamp[p] = ns;
+  }
+  taken = __reduce_add_sync(WARP_FULL, taken);
+  if (lane_id() == 0 && taken)
+    atomicAdd(accepted, (unsigned long long)taken);
 }
 
 // Loop-trip cap reached (WAVE_TRIP_CAP): the first warp to report writes the
@@ -641,17 +755,11 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
 // End of a wave: adaptive variance update (pathtracer.cpp:1129-1139), ray
 // totals, and the wave index for the next replay.
 __global__ void __launch_bounds__(256) k_wave_end(const RenderConst *__restrict__ rcp, Accum acc, WaveCounters wc,
-    uint32_t npix, int adaptive, int max_iter, unsigned long long *ray_totals)
+    uint32_t npix, int adaptive, int max_iter, unsigned long long *ray_totals, int samples)
 {
   if (adaptive) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
-      const float4 a = acc.acc[i], s = acc.start[i];
-      const V3 sv = V3{a.x, a.y, a.z} - V3{s.x, s.y, s.z};
-      float4 q = acc.acc_sq[i];
-      q.x = q.x + sv.x * sv.x;
-      q.y = q.y + sv.y * sv.y;
-      q.z = q.z + sv.z * sv.z;
-      acc.acc_sq[i] = q;
+      acc.acc_sq[i] = adapt_square(acc.acc_sq[i], acc.acc[i], acc.start[i]);
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -660,7 +768,8 @@ __global__ void __launch_bounds__(256) k_wave_end(const RenderConst *__restrict_
       cr += wc.count[k];
       sr += wc.scount[k];
     }
-    ray_totals[0] += wc.count[0];
+    if (samples)
+      ray_totals[0] += wc.count[0];
     ray_totals[1] += cr;
     ray_totals[2] += sr;
     *wc.wave += 1u;
@@ -737,9 +846,16 @@ __global__ void __launch_bounds__(256) k_read(Frame fr, uint32_t npix, float inv
 // ------------------------------------------------------------- launchers
 
 void launch_raygen(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, PathSoA out, Accum acc,
-    WaveCounters wc)
+    WaveCounters wc, AdaptState ad)
 {
-  k_raygen<<<c.blocks_raygen, 256, 0, s>>>(rc, sc, out, acc, wc);
+  k_raygen<<<c.blocks_raygen, 256, 0, s>>>(rc, sc, out, acc, wc, ad);
+}
+
+void launch_adapt_merge(cudaStream_t s, const RenderConst *rc, AdaptState ad, Accum lanes, WaveCounters wc,
+    uint32_t npix, uint32_t slots, int max_iter, uint64_t *accepted)
+{
+  k_adapt_merge<<<(npix + 255) / 256, 256, 0, s>>>(rc, ad, lanes, wc, npix, slots, max_iter,
+      (unsigned long long *)accepted);
 }
 
 void launch_trace(const LaunchCfg &c, cudaStream_t s, DevScene sc, PathSoA in, float4 *hits, WaveCounters wc, int it,
@@ -850,10 +966,11 @@ void launch_shadow_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, Shad
 }
 
 void launch_wave_end(cudaStream_t s, const RenderConst *rc, Accum acc, WaveCounters wc, uint32_t npix, int adaptive,
-    int max_iter, uint64_t *ray_totals)
+    int max_iter, uint64_t *ray_totals, bool samples)
 {
   const uint32_t blocks = adaptive ? (npix + 255) / 256 : 1u;
-  k_wave_end<<<blocks, 256, 0, s>>>(rc, acc, wc, npix, adaptive, max_iter, (unsigned long long *)ray_totals);
+  k_wave_end<<<blocks, 256, 0, s>>>(rc, acc, wc, npix, adaptive, max_iter, (unsigned long long *)ray_totals,
+      samples ? 1 : 0);
 }
 
 void launch_resolve(cudaStream_t s, Accum acc, Frame fr, uint32_t npix, uint32_t lanes, float weight, int first)

@@ -35,8 +35,12 @@ struct RenderConst {
   float tp_clamp;
   int32_t max_diffuse, max_glossy, max_transmission, max_volume;
   float clamp_direct, clamp_indirect;
-  uint32_t lanes; // samples of one pixel in flight per wave
+  uint32_t lanes; // samples of one pixel in flight per wave (adaptive sampling: see AdaptState)
 };
+
+// Samples every pixel takes before the variance gate may stop it
+// (pathtracer.cpp:710-725).
+constexpr uint32_t ADAPT_MIN_SAMPLES = 16;
 
 // Path state, structure of arrays over `cap` slots (two copies, ping-pong).
 struct PathSoA {
@@ -62,6 +66,24 @@ struct Accum {
   uint32_t *nsamp;  // samples started
   float4 *aov_n;    // normal.xyz, depth
   float4 *aov_a;    // albedo.xyz, (sample index + 1) of the write as float bits, 0 unwritten
+};
+
+// Adaptive sampling with several samples of a pixel in flight.  Whether a
+// pixel takes its next sample depends on the samples before it, and so does
+// the rounding of its running sums; but what a sample's path does depends only
+// on its pixel and sample index.  A wave therefore traces the next samples of
+// every pixel that may need them side by side (slot = sample in wave * npix +
+// pixel), with one accumulator plane per bounce iteration and kind of
+// contribution (shading, shadow ray) in which a path's contribution stands
+// alone, and k_adapt_merge then applies them pixel by pixel, sample by sample
+// and bounce by bounce to the pixel's state below, with the gate before each
+// sample, exactly as one sample per wave would have; samples the gate turns
+// out to refuse are dropped.
+struct AdaptState {
+  float4 *acc, *sq, *start; // per pixel: sums, squared sample values, sums when its last sample began
+  uint32_t *nsamp;          // per pixel: samples taken
+  float4 *aov_n, *aov_a;    // per pixel, as Accum's
+  float4 *planes;           // [2 * max_iter][slots]: shading and shadow contributions of each iteration
 };
 
 // Device counters of one wave.
@@ -189,7 +211,12 @@ void launch_shadow_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, Shad
     int refill, bool volumes);
 
 void launch_raygen(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, PathSoA out, Accum acc,
-    WaveCounters wc);
+    WaveCounters wc, AdaptState ad = AdaptState{});
+// End of an adaptive wave with several samples in flight: applies its samples
+// to the pixels' state and clears what they wrote.  lanes: the slots' aov
+// arrays; slots: their number; accepted: the samples taken are added to it.
+void launch_adapt_merge(cudaStream_t s, const RenderConst *rc, AdaptState ad, Accum lanes, WaveCounters wc,
+    uint32_t npix, uint32_t slots, int max_iter, uint64_t *accepted);
 // refill: a warp takes new rays once at least this many of its lanes are
 // idle (32: only when all are).  hq.hitq != nullptr: also write the hit and
 // miss index queues.
@@ -227,8 +254,9 @@ void launch_material_sort_batch(const LaunchCfg &c, cudaStream_t s, BatchTable b
 // Occlusion only: unoccluded rays keep tmax >= 0, occluded ones get tmax < 0.
 void launch_shadow_deferred(const LaunchCfg &c, cudaStream_t s, DevScene sc, ShadowSoA sh, WaveCounters wc, int it,
     int refill);
+// samples: add the wave's paths to the sample total (ray_totals[0]).
 void launch_wave_end(cudaStream_t s, const RenderConst *rc, Accum acc, WaveCounters wc, uint32_t npix, int adaptive,
-    int max_iter, uint64_t *ray_totals);
+    int max_iter, uint64_t *ray_totals, bool samples = true);
 void launch_resolve(cudaStream_t s, Accum acc, Frame fr, uint32_t npix, uint32_t lanes, float weight, int first);
 void launch_read(cudaStream_t s, Frame fr, uint32_t npix, float inv_samples, int channel, float *out);
 // Resident blocks per SM of a kernel (0 trace, 1 shade, 2 shadow, 3 raygen).
