@@ -1086,12 +1086,14 @@ struct AdjQueues {
 AdjQueues adj_queues(phc_renderer *r, size_t slots)
 {
   const size_t f4 = slots * 16;
-  const size_t per_path = 6 * f4, per_shadow = 5 * f4 + slots * 4 + 256;
-  ck(r->adj_pool.ensure(2 * per_path + per_shadow + f4 + 1024), "alloc adjoint queues");
+  auto padded = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+  // 6 fields of each path queue, 5 of the shadow queue and its 4-byte links,
+  // the collected radiance
+  ck(r->adj_pool.ensure((2 * 6 + 5 + 1) * padded(f4) + padded(slots * 4)), "alloc adjoint queues");
   char *p = r->adj_pool.as<char>();
   auto take = [&](size_t bytes) {
     char *q = p;
-    p += (bytes + 255) & ~size_t(255);
+    p += padded(bytes);
     return q;
   };
   AdjQueues a;
