@@ -1108,8 +1108,8 @@ __global__ void __launch_bounds__(128, PHC_ADJ_MIN_BLOCKS) k_adj_shade(const Ren
   __shared__ float svol[MAX_VOLUMES * 4];
   Grads g = begin_grads(smat, svol, sc, a);
   const RenderConst &rc = *rcp;
-  const uint32_t n = wc.count[it];
-  uint32_t *fetch = wc.fetch + 4 * it + 1;
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
+  uint32_t *fetch = wc.at(WaveCounters::F_SHADE, it);
   for (;;) {
     const uint32_t base = warp_fetch(fetch);
     if (base >= n)
@@ -1121,13 +1121,13 @@ __global__ void __launch_bounds__(128, PHC_ADJ_MIN_BLOCKS) k_adj_shade(const Ren
     if (j < n) {
       uint32_t i = j;
       if (hq.hitq) {
-        const uint32_t hc = wc.hcount[it];
+        const uint32_t hc = *wc.at(WaveCounters::HCOUNT, it);
         const bool sorted = hq.sorted != nullptr && hq.sort_threshold != 0u && hc >= hq.sort_threshold;
         i = j < hc ? (sorted ? hq.sorted[j] : hq.hitq[j]) : hq.missq[j - hc];
       }
       adj_shade_path(rc, sc, in, i, hits[i], it, a, g, cont, nx, has_sh, sr);
     }
-    const uint32_t o = warp_append(wc.count + it + 1, cont);
+    const uint32_t o = warp_append(wc.at(WaveCounters::COUNT, it + 1), cont);
     if (cont) {
       out.p.ray_o[o] = nx.o;
       out.p.ray_d[o] = nx.d;
@@ -1141,7 +1141,7 @@ __global__ void __launch_bounds__(128, PHC_ADJ_MIN_BLOCKS) k_adj_shade(const Ren
         put_vtx(out.v, o, nx.vq, nx.vmat);
       }
     }
-    const uint32_t so = warp_append(wc.scount + it, has_sh);
+    const uint32_t so = warp_append(wc.at(WaveCounters::SCOUNT, it), has_sh);
     if (has_sh) {
       sh.s.a[so] = sr.a;
       sh.s.b[so] = sr.b;
@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(128) k_adj_resolve(const RenderConst *__restri
   __shared__ float smat[MAX_SMEM_MATERIALS * NP];
   __shared__ float svol[MAX_VOLUMES * 4];
   Grads g = begin_grads(smat, svol, sc, a);
-  const uint32_t n = wc.scount[it];
+  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   const uint32_t npix = rcp->npix;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 s4 = sh.s.a[i];

@@ -112,6 +112,11 @@ struct phc_renderer {
   // frame (RenderBridge.cpp:424-435)
   Buf f_color, f_normal, f_albedo, read_buf;
   uint32_t width{0}, height{0}, samples{0}, sample_counter{0};
+  // streams beside `stream` for the independent kernels of a wave, and the
+  // events that fork and join them
+  static constexpr int SIDES = 3;
+  cudaStream_t side[SIDES]{};
+  cudaEvent_t fork_ev[SIDES]{}, join_ev[SIDES]{};
   // graph of one wave
   cudaGraphExec_t graph{nullptr};
   uint64_t graph_key[8]{};
@@ -134,6 +139,14 @@ struct phc_renderer {
       cudaEventDestroy(ev0);
     if (ev1)
       cudaEventDestroy(ev1);
+    for (int k = 0; k < SIDES; ++k) {
+      if (fork_ev[k])
+        cudaEventDestroy(fork_ev[k]);
+      if (join_ev[k])
+        cudaEventDestroy(join_ev[k]);
+      if (side[k])
+        cudaStreamDestroy(side[k]);
+    }
     if (stream)
       cudaStreamDestroy(stream);
   }
@@ -313,15 +326,7 @@ WaveCounters wave_counters(phc_renderer *r, int max_iter)
 {
   uint32_t *c = r->counters.as<uint32_t>();
   WaveCounters wc;
-  wc.count = c;
-  wc.scount = c + (max_iter + 1);
-  wc.hcount = c + (2 * max_iter + 1);
-  wc.mcount = c + (3 * max_iter + 1);
-  wc.fetch = c + (4 * max_iter + 1);
-  wc.vfetch = c + (8 * max_iter + 1);
-  wc.cfetch = c + (10 * max_iter + 1);
-  wc.vcount = c + ((10 + SHADE_CLASSES) * max_iter + 1);
-  wc.vqfetch = c + ((11 + SHADE_CLASSES) * max_iter + 1);
+  wc.base = c;
   wc.wave = c + wave_counter_words(max_iter);
   wc.error = c + wave_counter_words(max_iter) + 1;
   wc.dbg = c + wave_counter_words(max_iter) + 4;
@@ -373,7 +378,52 @@ struct KernelTimer {
   }
 };
 
+// Launches that may run beside what the main stream launches next: begin()
+// gives the stream for them, ordered after the main stream's launches so far;
+// end() marks their end, and join() makes the main stream's next launches wait
+// for them.  Off (on = false): everything on the main stream.
+class SideBranch {
+public:
+  SideBranch(phc_renderer *r, cudaStream_t main, int k, bool on) : r_(r), main_(main), k_(k), on_(on) {}
+  cudaStream_t begin()
+  {
+    if (!on_)
+      return main_;
+    ck(cudaEventRecord(r_->fork_ev[k_], main_), "fork");
+    ck(cudaStreamWaitEvent(r_->side[k_], r_->fork_ev[k_], 0), "fork");
+    return r_->side[k_];
+  }
+  void end()
+  {
+    if (!on_)
+      return;
+    ck(cudaEventRecord(r_->join_ev[k_], r_->side[k_]), "join");
+    open_ = true;
+  }
+  void join()
+  {
+    if (open_)
+      ck(cudaStreamWaitEvent(main_, r_->join_ev[k_], 0), "join");
+    open_ = false;
+  }
+
+private:
+  phc_renderer *r_;
+  cudaStream_t main_;
+  int k_;
+  bool on_, open_{false};
+};
+
 // One wave: counter reset, raygen, per iteration trace / shade / shadow, end.
+// An iteration's shadow rays only add to the accumulators, so they run beside
+// the next iteration's closest-hit rays (and volume tracking) and are joined
+// before its shading; the kernels that shade one iteration's paths (hits by
+// class, misses, scattering paths) share nothing but the output queues'
+// counters and run beside one another.  Each kernel of a wave ends with a few
+// long paths on an otherwise empty GPU; the next one fills it.  Measured
+// against one stream: 640 x 360, 1-spp frame of the 500K scene 1.40 -> 1.06 ms,
+// adaptive volume frame 25.8 -> 21.2 ms, adjoint of the differentiable workload
+// 10.8 -> 10.0 ms; frames of 2^27 paths lose nothing.
 // Returns the number of kernel launches.
 // wave_paths: paths of one wave (lanes x pixels); the material sort and the
 // class kernels are recorded only where an iteration can reach the sort
@@ -384,7 +434,7 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
     size_t wave_paths, int max_iter, int adaptive, bool counting, const AdaptState &ad, KernelTimer *tm = nullptr)
 {
   const WaveCounters wc = wave_counters(r, max_iter);
-  ck(cudaMemsetAsync(wc.count, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
+  ck(cudaMemsetAsync(wc.base, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
   const DevScene sc = r->scene.dev;
   const Accum acc_all = accum(r);
   const ShadowSoA sh{r->sh_a.as<float4>(), r->sh_b.as<float4>(), r->sh_c.as<float4>()};
@@ -438,10 +488,14 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
     hq.classes = classes ? 1u : 0u;
     ck(cudaMemsetAsync(r->sort_bins.p, 0, size_t(max_iter) * bin_words * 4, s), "reset sort bins");
   }
+  // without surfaces that let a path pass, the iteration at the depth limit
+  // casts no shadow rays (and is the last, render_const)
+  const int last_shadow = r->scene.may_pass ? max_iter : max_iter - 1;
   uint64_t launches = 2;
   if (tm)
     tm->begin_wave();
   timed(0, [&] { launch_raygen(cfg, s, rc, sc, path_soa(r, 0), acc_all, wc, ad); });
+    SideBranch shadows(r, s, 0, tm == nullptr), part_a(r, s, 1, tm == nullptr), part_b(r, s, 2, tm == nullptr);
   for (int it = 0; it < max_iter; ++it) {
     const PathSoA in = path_soa(r, it & 1), out = path_soa(r, (it + 1) & 1);
     float4 *hits = r->hits.as<float4>();
@@ -456,10 +510,14 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
     timed(1, [&] {
       launch_trace(cfg, s, sc, in, hits, wc, it, counting ? stats + 3 : nullptr, tu.trace_refill, hq_trace);
     });
-    if (vsplit) {
+    launches += 1;
+    if (vol_pre) {
       timed(5, [&] { launch_vol_scatter(cfg, s, rc, sc, in, hits, wc, it, hq, counting ? stats + 7 : nullptr); });
+      launches += 1;
+    }
+    if (vsplit) {
       timed(5, [&] { launch_vol_route(cfg, s, hits, wc, it, hq); });
-      launches += 2;
+      launches += 1;
     }
     if (sort) {
       timed(2, [&] {
@@ -467,37 +525,45 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
       });
       launches += 3;
     }
-    if (split) {
-      HitQueues hqi = hq;
-      if (classes) // the scatter leaves each bin's end in the upper half of the iteration's bins
-        hqi.cls_end = r->sort_bins.as<uint32_t>() + size_t(it) * bin_words + MAT_SORT_BINS;
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 1}, hqi); });
+    shadows.join(); // the last iteration's, which write the accumulators and read the shadow queue
+    HitQueues hqi = hq;
+    if (classes) // the scatter leaves each bin's end in the upper half of the iteration's bins
+      hqi.cls_end = r->sort_bins.as<uint32_t>() + size_t(it) * bin_words + MAT_SORT_BINS;
+    auto shade = [&](cudaStream_t on, int part) {
+      timed(2, [&] { launch_shade(cfg, on, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, part}, hqi); });
+      launches += 1;
+    };
+    if (split || vsplit) {
+      const cudaStream_t sa = part_a.begin();
+      shade(sa, 2);
+      if (vsplit)
+        shade(sa, 3);
       if (classes) {
+        const cudaStream_t sb = part_b.begin();
         for (uint32_t c = 1; c < SHADE_CLASSES; ++c)
-          timed(2, [&] { launch_shade_class(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, c, hqi); });
+          timed(2, [&] { launch_shade_class(cfg, c & 1u ? sb : s, rc, sc, in, out, hits, sh, ac, wc, it, c, hqi); });
         launches += SHADE_CLASSES - 1;
+        part_b.end();
       }
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 2}, hqi); });
-      launches += 4;
-    } else if (vsplit) {
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 3}, hq); });
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 1}, hq); });
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 2}, hq); });
-      launches += 3;
+      shade(s, 1);
+      part_a.end();
+      part_a.join();
+      part_b.join();
     } else {
-      if (vol_pre) {
-        timed(5, [&] { launch_vol_scatter(cfg, s, rc, sc, in, hits, wc, it, hq, counting ? stats + 7 : nullptr); });
-        launches += 1;
-      }
-      timed(2, [&] { launch_shade(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, ShadeVariant{full, 0}, hq); });
-      launches += 3;
+      shade(s, 0);
     }
-    timed(3, [&] { launch_shadow(cfg, s, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 5 : nullptr, tu.trace_refill); });
+    if (it == last_shadow)
+      continue;
+    const cudaStream_t ss = shadows.begin();
+    timed(3, [&] { launch_shadow(cfg, ss, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 5 : nullptr, tu.trace_refill); });
+    launches += 1;
     if (sc.volume_count > 0) {
-      timed(6, [&] { launch_shadow_volume(cfg, s, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 7 : nullptr); });
+      timed(6, [&] { launch_shadow_volume(cfg, ss, rc, sc, sh, ac_shadow, wc, it, counting ? stats + 7 : nullptr); });
       launches += 1;
     }
+    shadows.end();
   }
+  shadows.join();
   if (ad.planes) {
     timed(4, [&] {
       launch_adapt_merge(s, rc, ad, acc_all, wc, npix, uint32_t(wave_paths), max_iter, stats);
@@ -568,7 +634,7 @@ void validate_call(phc_renderer *r, const phc_settings &st)
 
 // The constants of one render call of a w x h frame (everything but the
 // sample offset and lanes); a background image goes to `bg`.
-RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg, cudaStream_t s)
+RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg, bool may_pass, cudaStream_t s)
 {
   const uint32_t w = st.width, h = st.height;
   const uint32_t npix = w * h;
@@ -579,7 +645,10 @@ RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg,
   rc.npix = npix;
   rc.spp = std::max<uint32_t>(st.pixel_samples, 1);
   rc.max_depth = std::max<uint32_t>(st.max_depth, 1);
-  rc.max_iter = rc.max_depth + 1u + 8u;
+  // every iteration is a bounce, or a passage through a surface (at most 8)
+  // where the scene has such surfaces: otherwise the 8 iterations past the
+  // depth limit have no paths and are left out
+  rc.max_iter = rc.max_depth + 1u + (may_pass ? 8u : 0u);
   std::memcpy(rc.bg, st.background, sizeof(rc.bg));
   // background image (RenderBridge.cpp:848-870)
   const size_t bg_n = size_t(st.background_width) * st.background_height * 4;
@@ -659,7 +728,7 @@ JobPlan prepare_job(phc_renderer *r, const phc_camera &cam, const phc_settings &
     r->height = h;
     reset = true;
   }
-  RenderConst rc = render_const(cam, st, r->bg_buf, s);
+  RenderConst rc = render_const(cam, st, r->bg_buf, r->scene.may_pass, s);
   rc.sample_offset = r->sample_counter;
   // samples of one pixel in flight: enough paths to fill the GPU
   const Tuning &tu = tuning();
@@ -903,7 +972,7 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
 {
   const Tuning &tu = tuning();
   const WaveCounters wc = wave_counters(lead, max_iter);
-  ck(cudaMemsetAsync(wc.count, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
+  ck(cudaMemsetAsync(wc.base, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
   const ShadowSoA sh{lead->sh_a.as<float4>(), lead->sh_b.as<float4>(), lead->sh_c.as<float4>(),
       lead->sh_job.as<uint32_t>()};
   const bool full = (features & (SCENE_VOLUMES | SCENE_SOURCES | SCENE_LIGHTS)) != 0 || !tu.shade_lean;
@@ -922,26 +991,37 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
   }
   float4 *hits = lead->hits.as<float4>();
   launch_raygen_batch(cfg, s, bt, path_soa(lead, 0), wc);
+  SideBranch shadows(lead, s, 0, true), part_a(lead, s, 1, true), part_b(lead, s, 2, true); // as in record_wave
   for (int it = 0; it < max_iter; ++it) {
     const PathSoA in = path_soa(lead, it & 1), out = path_soa(lead, (it + 1) & 1);
     launch_trace_batch(cfg, s, bt, in, hits, wc, it, tu.trace_refill, hq);
     if (sort)
       launch_material_sort_batch(cfg, s, bt, in.info, hits, hq, wc, it,
           lead->sort_bins.as<uint32_t>() + size_t(it) * bin_words);
+    shadows.join();
     if (split) {
       HitQueues hqi = hq;
       if (classes) // the scatter leaves each bin's end in the upper half of the iteration's bins
         hqi.cls_end = lead->sort_bins.as<uint32_t>() + size_t(it) * bin_words + MAT_SORT_BINS;
-      launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 1}, hqi);
-      if (classes)
+      const cudaStream_t sa = part_a.begin();
+      launch_shade_batch(cfg, sa, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 2}, hqi);
+      if (classes) {
+        const cudaStream_t sb = part_b.begin();
         for (uint32_t c = 1; c < SHADE_CLASSES; ++c)
-          launch_shade_class_batch(cfg, s, bt, in, out, hits, sh, wc, it, c, hqi);
-      launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 2}, hqi);
+          launch_shade_class_batch(cfg, c & 1u ? sb : s, bt, in, out, hits, sh, wc, it, c, hqi);
+        part_b.end();
+      }
+      launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 1}, hqi);
+      part_a.end();
+      part_a.join();
+      part_b.join();
     } else {
       launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 0}, hq);
     }
-    launch_shadow_batch(cfg, s, bt, sh, wc, it, tu.trace_refill, (features & SCENE_VOLUMES) != 0);
+    launch_shadow_batch(cfg, shadows.begin(), bt, sh, wc, it, tu.trace_refill, (features & SCENE_VOLUMES) != 0);
+    shadows.end();
   }
+  shadows.join();
   launch_wave_end(s, nullptr, Accum{}, wc, 0, 0, max_iter, lead->stats_buf.as<uint64_t>());
 }
 
@@ -1136,7 +1216,7 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
     throw ApiError(PHC_ERR_LIMIT, "volume gradients for more than PHC_ADJ_MAX_VOLUMES volumes");
   check_device(r);
   cudaStream_t s = r->stream;
-  const RenderConst base = render_const(cam, st, r->adj_bg, s);
+  const RenderConst base = render_const(cam, st, r->adj_bg, r->scene.may_pass, s);
   const uint32_t npix = base.npix, spp = base.spp;
   const int max_iter = int(base.max_iter);
   // both passes run over chunks of `chunk` samples, one sample per
@@ -1199,7 +1279,7 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
     ck(cudaMemsetAsync(wc.wave, 0, 8, s), "reset wave");
     record_wave(r, s, cfg, drc, npix, size_t(cnt) * npix, max_iter, 0, false, AdaptState{});
     // pass 2: the replay, bounce by bounce
-    ck(cudaMemsetAsync(wc.count, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
+    ck(cudaMemsetAsync(wc.base, 0, per_wave_counter_bytes(max_iter), s), "reset counters");
     ck(cudaMemsetAsync(wc.wave, 0, 4, s), "reset wave");
     ck(cudaMemsetAsync(q.collected, 0, size_t(cnt) * npix * 16, s), "reset adjoint");
     launch_raygen(cfg, s, drc, sc, q.path[0].p, accum(r), wc);
@@ -1213,16 +1293,23 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
       rq.sort_threshold = uint32_t(tu.sort_threshold);
       ck(cudaMemsetAsync(r->sort_bins.p, 0, size_t(max_iter) * bin_words * 4, s), "reset sort bins");
     }
+    // a bounce's shadow rays and their vertices' gradients run beside the next
+    // bounce's closest-hit rays and sort; they write the next queue's remainders
+    SideBranch shadows(r, s, 0, true);
     for (int it = 0; it < max_iter; ++it) {
       const AdjPathSoA &in = q.path[it & 1], &out = q.path[(it + 1) & 1];
       float4 *hits = r->hits.as<float4>();
       launch_trace(cfg, s, sc, in.p, hits, wc, it, nullptr, tu.trace_refill, rq);
       if (rq.hitq)
         launch_material_sort(cfg, s, sc, hits, rq, wc, it, r->sort_bins.as<uint32_t>() + size_t(it) * bin_words);
+      shadows.join();
       launch_adj_shade(acfg, s, drc, sc, in, out, hits, q.shadow, wc, it, a, rq);
-      launch_shadow_deferred(cfg, s, sc, q.shadow.s, wc, it, tu.trace_refill);
-      launch_adj_resolve(acfg, s, drc, sc, q.shadow, out, wc, it, a);
+      const cudaStream_t ss = shadows.begin();
+      launch_shadow_deferred(cfg, ss, sc, q.shadow.s, wc, it, tu.trace_refill);
+      launch_adj_resolve(acfg, ss, drc, sc, q.shadow, out, wc, it, a);
+      shadows.end();
     }
+    shadows.join();
     launch_adj_finish(s, r->sm_count * 8, uint32_t(size_t(cnt) * npix), a);
     ck(cudaGetLastError(), "adjoint kernels");
   }
@@ -1383,6 +1470,11 @@ int phc_create(phc_renderer **out)
     ck(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     ck(cudaEventCreate(&r->ev0), "cudaEventCreate");
     ck(cudaEventCreate(&r->ev1), "cudaEventCreate");
+    for (int k = 0; k < phc_renderer::SIDES; ++k) {
+      ck(cudaStreamCreateWithFlags(&r->side[k], cudaStreamNonBlocking), "cudaStreamCreate");
+      ck(cudaEventCreateWithFlags(&r->fork_ev[k], cudaEventDisableTiming), "cudaEventCreate");
+      ck(cudaEventCreateWithFlags(&r->join_ev[k], cudaEventDisableTiming), "cudaEventCreate");
+    }
   });
   if (rc != PHC_OK) {
     delete r;

@@ -122,6 +122,21 @@ uint32_t shade_class_of(uint32_t lobes)
   return 0u;
 }
 
+// Whether a path may leave a surface of this material without having made a
+// bounce: surfaces hidden to the camera and stochastic transparency (an alpha
+// below 1, resolve_material).  Opacity from an attribute, a sampler or a
+// texture counts as below 1.
+bool material_may_pass(const DevMaterial &m)
+{
+  if (m.flags & MF_HIDDEN)
+    return true;
+  if (m.alpha_mode == 1)
+    return false;
+  if (m.src_kind[SRC_ALPHA] != 0 || m.base_color_alpha || m.alpha_tex >= 0 || m.base_tex >= 0)
+    return true;
+  return !(m.alpha_mode == 2 ? m.alpha >= m.alpha_cutoff : m.alpha >= 1.f);
+}
+
 // photon::pt::Material{} defaults (material.h:35-82), used when the scene has
 // no material at all (RenderBridge.cpp:518-519).
 DevMaterial default_material()
@@ -1315,6 +1330,9 @@ std::string DeviceScene::upload(const HostScene &h, cudaStream_t s)
   for (const DevMaterial &m : h.materials)
     class_mask |= 1u << (m.shade_class % SHADE_CLASSES);
   shade_class_count = uint32_t(__builtin_popcount(class_mask));
+  may_pass = false;
+  for (const DevMaterial &m : h.materials)
+    may_pass = may_pass || material_may_pass(m);
   table_floats[PHC_TABLE_MAJORANTS] = h.vol_majorants.size();
   table_floats[PHC_TABLE_ENV_MARGINAL] = h.env_marginal.size();
   table_floats[PHC_TABLE_ENV_CONDITIONAL] = h.env_conditional.size();

@@ -130,6 +130,7 @@ struct DeviceScene {
   uint64_t node_bytes{0}, tri_bytes{0};
   uint64_t texel_count{0};
   uint32_t shade_class_count{0}; // distinct shading classes among the materials
+  bool may_pass{true};           // a path may go through a surface without a bounce (scene_may_pass)
   uint32_t bvh_depth{0};
   uint64_t table_floats[5]{}; // lengths of the tables phc_scene_table reads (PHC_TABLE_*)
   ~DeviceScene();

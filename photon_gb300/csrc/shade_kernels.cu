@@ -22,8 +22,8 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
   // once wc.vol_refill lanes of its warp are idle; every trip is at most
   // wc.vol_passes passes of every busy lane's tracking (vt_pass: a macro-cell
   // step or a density lookup), ending at its next lookup
-  const uint32_t n = wc.count[it];
-  uint32_t *fetch = wc.vfetch + 2 * it;
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
+  uint32_t *fetch = wc.at(WaveCounters::F_VSCATTER, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
@@ -93,20 +93,20 @@ __global__ void __launch_bounds__(256) k_vol_route(const float4 *__restrict__ hi
 {
   if (wave_failed(wc))
     return;
-  const uint32_t n = wc.count[it];
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   const uint32_t warps = gridDim.x * (blockDim.x / 32u);
   for (uint32_t base = (blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5)) * 32u; base < n; base += warps * 32u) {
     const uint32_t i = base + lane_id();
     uint32_t route = 0u;
     if (i < n)
       route = hq.vscatter[i].x >= 0.f ? 1u : (__float_as_uint(hits[i].y) != 0xffffffffu ? 2u : 3u);
-    const uint32_t a = warp_append(wc.vcount + it, route == 1u);
+    const uint32_t a = warp_append(wc.at(WaveCounters::VCOUNT, it), route == 1u);
     if (route == 1u)
       hq.vscatq[a] = i;
-    const uint32_t b = warp_append(wc.hcount + it, route == 2u);
+    const uint32_t b = warp_append(wc.at(WaveCounters::HCOUNT, it), route == 2u);
     if (route == 2u)
       hq.hitq[b] = i;
-    const uint32_t m = warp_append(wc.mcount + it, route == 3u);
+    const uint32_t m = warp_append(wc.at(WaveCounters::MCOUNT, it), route == 3u);
     if (route == 3u)
       hq.missq[m] = i;
   }

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
   if (wave_failed(wc))
     return;
   const uint32_t n_all =
-      PART == 0 ? wc.count[it] : (PART == 1 ? wc.hcount[it] : (PART == 2 ? wc.mcount[it] : wc.vcount[it]));
+      PART == 0 ? *wc.at(WaveCounters::COUNT, it) : (PART == 1 ? *wc.at(WaveCounters::HCOUNT, it) : (PART == 2 ? *wc.at(WaveCounters::MCOUNT, it) : *wc.at(WaveCounters::VCOUNT, it)));
   const bool sorted = PART == 1 && hq.sort_threshold != 0u && n_all >= hq.sort_threshold;
   uint32_t lo = 0, n = n_all;
   if (PART == 1 && hq.cls_end && sorted) {
@@ -370,8 +370,8 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
   } else if (CLS != 0) {
     return;
   }
-  uint32_t *fetch = CLS != 0 ? wc.cfetch + it * SHADE_CLASSES + CLS
-                             : (PART == 3 ? wc.vqfetch + it : wc.fetch + 4 * it + (PART == 2 ? 2 : 1));
+  uint32_t *fetch = CLS != 0 ? wc.at(WaveCounters::F_CLASS + CLS, it)
+                             : wc.at(PART == 3 ? WaveCounters::F_VSHADE : (PART == 2 ? WaveCounters::F_MISS : WaveCounters::F_SHADE), it);
   for (;;) {
     const uint32_t base = warp_fetch(fetch);
     if (base >= n)
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
       }
     }
     if (PART != 2) { // misses never continue nor cast shadow rays
-      const uint32_t o = warp_append(wc.count + it + 1, cont);
+      const uint32_t o = warp_append(wc.at(WaveCounters::COUNT, it + 1), cont);
       if (cont) {
         out.ray_o[o] = np.o;
         out.ray_d[o] = np.d;
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
         out.info[o] = make_uint4(np.info.x, np.info.y, np.info.z, np.info.w | job_bits);
         out.pdist[o] = np.pdist;
       }
-      const uint32_t so = warp_append(wc.scount + it, has_sh);
+      const uint32_t so = warp_append(wc.at(WaveCounters::SCOUNT, it), has_sh);
       if (has_sh) {
         sh.a[so] = sr.a;
         sh.b[so] = sr.b;

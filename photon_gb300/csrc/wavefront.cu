@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) k_raygen_batch(BatchTable bt, PathSoA out
       camera_ray(rc, pixel, sample_index, ro, rd, tmin, tmax);
       bt.jobs[job].acc.nsamp[slot] += 1u;
     }
-    const uint32_t o = warp_append(wc.count, live);
+    const uint32_t o = warp_append(wc.at(WaveCounters::COUNT, 0), live);
     if (live) {
       out.ray_o[o] = f4(ro, tmin);
       out.ray_d[o] = f4(rd, tmax);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ 
   if (dense) {
     const uint32_t live_lanes = s0 < rc.spp ? min(rc.lanes, rc.spp - s0) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
-      wc.count[0] = live_lanes * rc.npix;
+      *wc.at(WaveCounters::COUNT, 0) = live_lanes * rc.npix;
   }
   for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < total;
        base += gridDim.x * blockDim.x) {
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ 
         }
       }
     }
-    const uint32_t o = dense ? i : warp_append(wc.count, live);
+    const uint32_t o = dense ? i : warp_append(wc.at(WaveCounters::COUNT, 0), live);
     if (live) {
       out.ray_o[o] = f4(ro, tmin);
       out.ray_d[o] = f4(rd, tmax);
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) k_adapt_merge(const RenderConst *__restri
   const uint32_t s0 = *wc.wave * rc.lanes;
   const uint32_t cnt = s0 < rc.spp ? min(rc.lanes, rc.spp - s0) : 0u;
   int iters = 0; // iterations that had paths (or shadow rays, which come from paths)
-  while (iters < max_iter && wc.count[iters] != 0u)
+  while (iters < max_iter && *wc.at(WaveCounters::COUNT, iters) != 0u)
     ++iters;
   uint32_t taken = 0;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) k_adapt_merge(const RenderConst *__restri
             a.w = a.w + c.w;
           }
         }
-        if (wc.scount[it] != 0u) {
+        if (*wc.at(WaveCounters::SCOUNT, it) != 0u) {
           float4 *np = sp + slots;
           const float4 n = *np;
           if (!(n.x == 0.f && n.y == 0.f && n.z == 0.f)) {
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
 {
   if (wave_failed(wc))
     return;
-  const uint32_t n = wc.count[it];
-  uint32_t *fetch = wc.fetch + 4 * it;
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
+  uint32_t *fetch = wc.at(WaveCounters::F_TRACE, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
@@ -407,9 +407,9 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
       uint32_t hb = 0, mb = 0;
       if (lane == 0) {
         if (hm)
-          hb = atomicAdd(wc.hcount + it, uint32_t(__popc(hm)));
+          hb = atomicAdd(wc.at(WaveCounters::HCOUNT, it), uint32_t(__popc(hm)));
         if (mm)
-          mb = atomicAdd(wc.mcount + it, uint32_t(__popc(mm)));
+          mb = atomicAdd(wc.at(WaveCounters::MCOUNT, it), uint32_t(__popc(mm)));
       }
       hb = __shfl_sync(WARP_FULL, hb, 0);
       mb = __shfl_sync(WARP_FULL, mb, 0);
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256) k_mat_hist(DevScene sc, BatchTable bt, co
   if (wave_failed(wc))
     return;
   __shared__ uint32_t h[MAT_SORT_BINS];
-  const uint32_t n = wc.hcount[it];
+  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (n < hq.sort_threshold)
     return;
   for (uint32_t b = threadIdx.x; b < MAT_SORT_BINS; b += blockDim.x)
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(MAT_SORT_BINS) k_mat_scan(HitQueues hq, WaveCo
   if (wave_failed(wc))
     return;
   __shared__ uint32_t t[MAT_SORT_BINS];
-  if (wc.hcount[it] < hq.sort_threshold)
+  if (*wc.at(WaveCounters::HCOUNT, it) < hq.sort_threshold)
     return;
   const uint32_t b = threadIdx.x;
   t[b] = bins[b];
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(256) k_mat_scatter(DevScene sc, BatchTable bt,
   if (wave_failed(wc))
     return;
   __shared__ uint32_t cnt[MAT_SORT_BINS];
-  const uint32_t n = wc.hcount[it];
+  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (n < hq.sort_threshold)
     return;
   uint32_t *start = bins + MAT_SORT_BINS;
@@ -560,8 +560,8 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
 {
   if (wave_failed(wc))
     return;
-  const uint32_t n = wc.scount[it];
-  uint32_t *fetch = wc.fetch + 4 * it + 3;
+  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
+  uint32_t *fetch = wc.at(WaveCounters::F_SHADOW, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
@@ -678,8 +678,8 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
   // transmittance (stream dimension 0x10000 + iteration) times the NEE
   // contribution into the path's pixel slot; persistent warps with refill,
   // one tracking pass per busy lane and trip, as in k_vol_scatter
-  const uint32_t n = wc.scount[it];
-  uint32_t *fetch = wc.vfetch + 2 * it + 1;
+  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
+  uint32_t *fetch = wc.at(WaveCounters::F_VSHADOW, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
@@ -765,11 +765,11 @@ __global__ void __launch_bounds__(256) k_wave_end(const RenderConst *__restrict_
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     unsigned long long cr = 0, sr = 0;
     for (int k = 0; k < max_iter; ++k) {
-      cr += wc.count[k];
-      sr += wc.scount[k];
+      cr += *wc.at(WaveCounters::COUNT, k);
+      sr += *wc.at(WaveCounters::SCOUNT, k);
     }
     if (samples)
-      ray_totals[0] += wc.count[0];
+      ray_totals[0] += *wc.at(WaveCounters::COUNT, 0);
     ray_totals[1] += cr;
     ray_totals[2] += sr;
     *wc.wave += 1u;

@@ -86,25 +86,48 @@ struct AdaptState {
   float4 *planes;           // [2 * max_iter][slots]: shading and shadow contributions of each iteration
 };
 
-// Device counters of one wave.
+// Device counters of one wave, per bounce iteration, COUNTER_LINE words apart:
+// the warps of a launch append to and fetch from several of them at once, and
+// atomics to one line, or to lines of one L2 slice, take turns.  The box room's
+// frame (16.8M paths) with counters 1 / 8 / 16 / 32 / 64 / 256 words apart:
+// 12.4 / 10.0 / 9.2 / 9.7 / 9.1 / 8.7 ms, its closest-hit rays 3.76 / 2.99 / 2.31 /
+// 2.79 / 2.28 / 1.92 ms; with the queues appended 32 entries at a time (k_trace)
+// 64 and 256 words measure the same, and 64 words are 92 KB to clear per wave.
+constexpr uint32_t COUNTER_LINE = 64;
 struct WaveCounters {
-  uint32_t *count;   // [max_iter + 1] paths entering iteration it
-  uint32_t *scount;  // [max_iter] shadow rays of iteration it
-  uint32_t *hcount;  // [max_iter] closest-hit results that hit (split queues)
-  uint32_t *mcount;  // [max_iter] closest-hit results that missed (split queues)
-  uint32_t *fetch;   // [4 * max_iter] work counters: trace, shade (all/hits), shade misses, shadow
-  uint32_t *vfetch;  // [2 * max_iter] work counters: volume scattering, shadow transmittance
-  uint32_t *cfetch;  // [SHADE_CLASSES * max_iter] work counters of the class hit-shading kernels
-  uint32_t *vcount;  // [max_iter] paths that scatter in a volume (volume scenes, split queues)
-  uint32_t *vqfetch; // [max_iter] work counters of the shading of those paths
+  uint32_t *base;    // [(max_iter + 1) * COUNTERS] lines
   uint32_t *wave;    // current wave index within the render call
   uint32_t *error;   // sticky error word
   uint32_t *dbg;     // [WAVE_DBG_WORDS] record of the first self-check failure
   uint32_t trip_cap; // loop trips after which a persistent warp stops (tuning key wave_trip_cap)
   uint32_t vol_refill; // a volume-tracking warp takes new rays once this many lanes are idle (tuning key vol_refill)
   uint32_t vol_passes; // tracking passes per lane and loop trip at most (tuning key vol_passes)
+
+  enum : uint32_t {
+    COUNT,   // paths entering the iteration (one more than max_iter)
+    SCOUNT,  // shadow rays of the iteration
+    HCOUNT,  // closest-hit results that hit (split queues)
+    MCOUNT,  // closest-hit results that missed (split queues)
+    VCOUNT,  // paths that scatter in a volume (volume scenes, split queues)
+    F_TRACE, // work counters: trace, shade (all / hits), shade misses, shadow,
+    F_SHADE, // volume scattering, shadow transmittance, shading of scattering
+    F_MISS,  // paths, then the class hit-shading kernels (F_CLASS + class)
+    F_SHADOW,
+    F_VSCATTER,
+    F_VSHADOW,
+    F_VSHADE,
+    F_CLASS,
+    COUNTERS = F_CLASS + SHADE_CLASSES
+  };
+  __host__ __device__ uint32_t *at(uint32_t kind, int it) const
+  {
+    return base + (uint32_t(it) * COUNTERS + kind) * COUNTER_LINE;
+  }
 };
-inline size_t wave_counter_words(int max_iter) { return size_t((12 + SHADE_CLASSES) * max_iter + 1); }
+inline size_t wave_counter_words(int max_iter)
+{
+  return size_t(max_iter + 1) * WaveCounters::COUNTERS * COUNTER_LINE;
+}
 
 // Self-check of the persistent traversal loops: a warp that makes more than
 // WaveCounters::trip_cap loop trips (each trip is one traversal step of every
@@ -139,8 +162,8 @@ struct HitQueues {
   float4 *vscatter = nullptr;
   uint32_t *vrng = nullptr;
   // Volume scenes with split queues: after k_vol_scatter, k_vol_route puts
-  // every path in vscatq (it scatters in a volume; wc.vcount), hitq or missq
-  // (it reaches its surface hit / escapes; wc.hcount / wc.mcount), and the
+  // every path in vscatq (it scatters in a volume; WaveCounters::VCOUNT), hitq or missq
+  // (it reaches its surface hit / escapes; HCOUNT / MCOUNT), and the
   // closest-hit kernel writes no queue.
   uint32_t *vscatq = nullptr;
   // Sorting by shading class (lean scenes): bins are grouped per class
