@@ -602,9 +602,7 @@ void check_wave_error(uint32_t w, const WaveCounters &wc, cudaStream_t s)
           std::to_string(d[2]) + ", exhausted " + std::to_string(d[3]) + "; ray " + std::to_string(d[4]) + " o " +
           f(5) + " " + f(6) + " " + f(7) + " tmax " + f(8) + " d " + f(9) + " " + f(10) + " " + f(11) + " sp " +
           std::to_string(d[12]) + " base " + std::to_string(d[13]) + " hits " + std::to_string(d[14]) + " imask " +
-          std::to_string(d[15]) + " steps " + std::to_string(d[16]) + " rays of the lane " + std::to_string(d[17]) + "; warp fetch trips " + std::to_string(d[18]) +
-          " step trips " + std::to_string(d[19]) + " longest ray " + std::to_string(d[20]) + " steps (ray " +
-          std::to_string(d[21]) + "); trips " + std::to_string(d[22]) + " active " + std::to_string(d[23]) + ")");
+          std::to_string(d[15]) + "; trips " + std::to_string(d[16]) + " active " + std::to_string(d[17]) + ")");
 }
 
 // adapt_lanes: paths of an adaptive wave and the bytes of its accumulator planes

@@ -251,16 +251,10 @@ __global__ void __launch_bounds__(256) k_adapt_merge(const RenderConst *__restri
 // error word and its record (the state of its first busy lane).  Called by
 // every lane of the warp.
 __device__ __forceinline__ void record_cap(const WaveCounters &wc, uint32_t code, uint32_t n, uint32_t fetched,
-    bool busy, bool exhausted, uint32_t idx, float4 o, float4 d, const TravState &s, uint32_t steps, uint32_t rays,
-    uint32_t fetch_trips, uint32_t step_trips, uint32_t max_steps, uint32_t max_idx, uint32_t trips)
+    bool busy, bool exhausted, uint32_t idx, float4 o, float4 d, const TravState &s, uint32_t trips)
 {
   const uint32_t active = __activemask();
   const uint32_t bm = __ballot_sync(WARP_FULL, busy);
-  // the busy lane with the most steps on its current ray
-  uint32_t best = busy ? steps : 0u;
-  for (int off = 16; off > 0; off >>= 1)
-    best = max(best, __shfl_xor_sync(WARP_FULL, best, off));
-  const uint32_t cand = __ballot_sync(WARP_FULL, busy && steps == best);
   uint32_t won = 0;
   if (lane_id() == 0)
     won = atomicCAS(wc.error, 0u, code) == 0u ? 1u : 0u;
@@ -273,8 +267,10 @@ __device__ __forceinline__ void record_cap(const WaveCounters &wc, uint32_t code
     r[1] = fetched;
     r[2] = bm;
     r[3] = exhausted ? 1u : 0u;
+    r[16] = trips;
+    r[17] = active;
   }
-  if (cand != 0u && lane_id() == uint32_t(__ffs(int(cand)) - 1)) {
+  if (bm != 0u && lane_id() == uint32_t(__ffs(int(bm)) - 1)) {
     r[4] = idx;
     r[5] = __float_as_uint(o.x);
     r[6] = __float_as_uint(o.y);
@@ -287,22 +283,7 @@ __device__ __forceinline__ void record_cap(const WaveCounters &wc, uint32_t code
     r[13] = s.g_base;
     r[14] = s.g_hits;
     r[15] = s.g_imask;
-    r[16] = steps;
-    r[17] = rays;
   }
-  uint32_t ms = max_steps;
-  for (int off = 16; off > 0; off >>= 1)
-    ms = max(ms, __shfl_xor_sync(WARP_FULL, ms, off));
-  const uint32_t mc = __ballot_sync(WARP_FULL, max_steps == ms);
-  if (lane_id() == 0) {
-    r[18] = fetch_trips;
-    r[19] = step_trips;
-    r[20] = ms;
-    r[22] = trips;
-    r[23] = active;
-  }
-  if (lane_id() == uint32_t(__ffs(int(mc)) - 1))
-    r[21] = max_idx;
 }
 
 // ------------------------------------------------------------ closest hit
@@ -316,7 +297,7 @@ __device__ __forceinline__ void record_cap(const WaveCounters &wc, uint32_t code
 #define PHC_TRACE_MIN_BLOCKS 8 // 64 registers: 8 resident 128-thread blocks per SM
 #endif
 #ifndef PHC_TRACE_MIN_BLOCKS_INST
-#define PHC_TRACE_MIN_BLOCKS_INST 8 // the two-level variant (more state: the world ray)
+#define PHC_TRACE_MIN_BLOCKS_INST 7 // the two-level variant (more state: the world ray)
 #endif
 // INST: the scene has instances (two-level traversal, trav_step2); the hit's
 // instance slot goes to hq.inst.
@@ -337,30 +318,35 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
   TravCounters ctr{0u, 0u};
   std::conditional_t<INST, TravState2, TravState> s;
   uint2 stack[PHC_STACK_SIZE];
-  bool busy = false, exhausted = false;
-  uint32_t idx = 0, steps = 0, rays = 0, fetch_trips = 0, step_trips = 0, max_steps = 0, max_idx = 0;
+  bool busy = false;
+  WarpFeed feed(n, per_warp);
+  uint32_t idx = 0;
   const uint4 *nodes = sc.nodes;
   const float4 *tris = sc.tris;
+  // SPLIT: the finished rays wait in the warp's ring buffers until a queue
+  // gets 32 of them at once (one atomic and one line instead of one per trip
+  // with a finished lane): 500K workload 83.2 -> 81.5 ms, and its shading, which
+  // reads the queues in their order, 48.9 -> 47.7 ms
+  __shared__ uint32_t out_rings[SPLIT ? 4 : 1][2][64];
+  auto &out = out_rings[SPLIT ? threadIdx.x >> 5 : 0];
+  uint32_t h_at = 0, h_n = 0, m_at = 0, m_n = 0;
   // The idle mask changes only when lanes finish or fetch, so the warp votes
   // (refill, queue appends) run only on trips where some lane finished.
   uint32_t idle = lanes_on;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) { // warp-uniform: every lane counts the same trips
-      record_cap(wc, (WAVE_ERR_TRACE << 16) | uint32_t(it), n, *fetch, busy, exhausted, idx, in.ray_o[idx],
-          in.ray_d[idx], s, steps, rays, fetch_trips, step_trips, max_steps, max_idx, trips);
+      record_cap(wc, (WAVE_ERR_TRACE << 16) | uint32_t(it), n, *fetch, busy, feed.empty(), idx, in.ray_o[idx],
+          in.ray_d[idx], s, trips);
       break;
     }
-    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
+    if (!feed.empty() && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
-      const uint32_t k = uint32_t(__popc(idle));
-      const uint32_t base = warp_fetch(fetch, k);
-      ++fetch_trips;
-      if (base + k >= n)
-        exhausted = true;
+      uint32_t k = uint32_t(__popc(idle));
+      const uint32_t base = feed.take(fetch, n, k);
       if ((idle >> lane) & 1u) {
-        const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
-        if (my < n) {
-          idx = my;
+        const uint32_t rank = uint32_t(__popc(idle & lt_mask));
+        if (rank < k) {
+          idx = base + rank;
           const float4 o = in.ray_o[idx], d = in.ray_d[idx];
           if (BATCH) { // the BVH of the path's job
             const BatchJob &job = bt.jobs[in.info[idx].w >> BATCH_JOB_SHIFT];
@@ -371,30 +357,22 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
             trav_init2(s, v3(o), v3(d), o.w, d.w);
           else
             trav_init(s, v3(o), v3(d), o.w, d.w);
-          steps = 0;
-          ++rays;
           busy = true;
         }
       }
       idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
     if (idle == lanes_on) {
-      if (exhausted)
+      if (feed.empty())
         break;
       continue;
     }
     bool done = false;
-    ++step_trips;
     if (busy) {
       if constexpr (INST)
         done = !trav_step2<false, COUNT>(nodes, tris, sc.inst_w2o, sc.inst_info, s, stack, &ctr);
       else
         done = !trav_step<false, COUNT>(nodes, tris, s, stack, &ctr);
-      ++steps;
-      if (steps > max_steps) {
-        max_steps = steps;
-        max_idx = idx;
-      }
     }
     __syncwarp(); // every lane back from the step's divergent work before the vote
     const uint32_t dm = __ballot_sync(WARP_FULL, done);
@@ -404,20 +382,20 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
       const bool is_hit = done && s.best.prim != 0xffffffffu;
       const uint32_t hm = __ballot_sync(WARP_FULL, is_hit);
       const uint32_t mm = dm & ~hm;
-      uint32_t hb = 0, mb = 0;
-      if (lane == 0) {
-        if (hm)
-          hb = atomicAdd(wc.at(WaveCounters::HCOUNT, it), uint32_t(__popc(hm)));
-        if (mm)
-          mb = atomicAdd(wc.at(WaveCounters::MCOUNT, it), uint32_t(__popc(mm)));
+      if (done)
+        out[is_hit ? 0 : 1][((is_hit ? h_at + h_n : m_at + m_n) + uint32_t(__popc((is_hit ? hm : mm) & lt_mask))) & 63u] = idx;
+      h_n += uint32_t(__popc(hm));
+      m_n += uint32_t(__popc(mm));
+      __syncwarp();
+      if (h_n >= 32u) {
+        hq.hitq[warp_fetch(wc.at(WaveCounters::HCOUNT, it), 32u) + lane] = out[0][(h_at + lane) & 63u];
+        h_at += 32u;
+        h_n -= 32u;
       }
-      hb = __shfl_sync(WARP_FULL, hb, 0);
-      mb = __shfl_sync(WARP_FULL, mb, 0);
-      if (done) {
-        if (is_hit)
-          hq.hitq[hb + uint32_t(__popc(hm & lt_mask))] = idx;
-        else
-          hq.missq[mb + uint32_t(__popc(mm & lt_mask))] = idx;
+      if (m_n >= 32u) {
+        hq.missq[warp_fetch(wc.at(WaveCounters::MCOUNT, it), 32u) + lane] = out[1][(m_at + lane) & 63u];
+        m_at += 32u;
+        m_n -= 32u;
       }
     }
     if (done) {
@@ -427,6 +405,19 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
       busy = false;
     }
     idle |= dm;
+  }
+  if (SPLIT) { // what is left in the buffers
+    __syncwarp();
+    if (h_n) {
+      const uint32_t base = warp_fetch(wc.at(WaveCounters::HCOUNT, it), h_n);
+      if (lane < h_n)
+        hq.hitq[base + lane] = out[0][(h_at + lane) & 63u];
+    }
+    if (m_n) {
+      const uint32_t base = warp_fetch(wc.at(WaveCounters::MCOUNT, it), m_n);
+      if (lane < m_n)
+        hq.missq[base + lane] = out[1][(m_at + lane) & 63u];
+    }
   }
   if (COUNT) {
     atomicAdd((unsigned long long *)&stats[0], (unsigned long long)ctr.nodes);
@@ -571,8 +562,9 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
   TravCounters ctr{0u, 0u};
   std::conditional_t<INST, TravState2, TravState> s;
   uint2 stack[PHC_STACK_SIZE];
-  bool busy = false, exhausted = false;
-  uint32_t idx = 0, job = 0, steps = 0, rays = 0, fetch_trips = 0, step_trips = 0, max_steps = 0, max_idx = 0;
+  bool busy = false;
+  WarpFeed feed(n, per_warp);
+  uint32_t idx = 0, job = 0;
   const uint4 *nodes = sc.nodes;
   const float4 *tris = sc.tris;
   // persistent warps with dynamic refill, as in k_trace: the idle mask
@@ -580,21 +572,18 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
   uint32_t idle = lanes_on;
   for (uint32_t trips = 0;; ++trips) {
     if (trips >= wc.trip_cap) {
-      record_cap(wc, (WAVE_ERR_SHADOW << 16) | uint32_t(it), n, *fetch, busy, exhausted, idx, sh.a[idx], sh.b[idx],
-          s, steps, rays, fetch_trips, step_trips, max_steps, max_idx, trips);
+      record_cap(wc, (WAVE_ERR_SHADOW << 16) | uint32_t(it), n, *fetch, busy, feed.empty(), idx, sh.a[idx], sh.b[idx],
+          s, trips);
       break;
     }
-    if (!exhausted && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
+    if (!feed.empty() && (idle == lanes_on || uint32_t(__popc(idle)) >= refill_at)) {
       __syncwarp();
-      const uint32_t k = uint32_t(__popc(idle));
-      const uint32_t base = warp_fetch(fetch, k);
-      ++fetch_trips;
-      if (base + k >= n)
-        exhausted = true;
+      uint32_t k = uint32_t(__popc(idle));
+      const uint32_t base = feed.take(fetch, n, k);
       if ((idle >> lane) & 1u) {
-        const uint32_t my = base + uint32_t(__popc(idle & lt_mask));
-        if (my < n) {
-          idx = my;
+        const uint32_t rank = uint32_t(__popc(idle & lt_mask));
+        if (rank < k) {
+          idx = base + rank;
           const float4 a = sh.a[idx], b = sh.b[idx];
           if (BATCH) {
             job = sh.job[idx];
@@ -605,26 +594,18 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
             trav_init2(s, v3(a), v3(b), 0.f, a.w);
           else
             trav_init(s, v3(a), v3(b), 0.f, a.w);
-          steps = 0;
-          ++rays;
           busy = true;
         }
       }
       idle = __ballot_sync(WARP_FULL, !busy) & lanes_on;
     }
     if (idle == lanes_on) {
-      if (exhausted)
+      if (feed.empty())
         break;
       continue;
     }
-    ++step_trips;
     bool more = true;
     if (busy) {
-      ++steps;
-      if (steps > max_steps) {
-        max_steps = steps;
-        max_idx = idx;
-      }
       if constexpr (INST)
         more = trav_step2<true, COUNT>(nodes, tris, sc.inst_w2o, sc.inst_info, s, stack, &ctr);
       else

@@ -140,8 +140,9 @@ __device__ __forceinline__ bool wave_failed(const WaveCounters &wc) { return *(v
 enum : uint32_t { WAVE_ERR_TRACE = 1u, WAVE_ERR_SHADOW = 2u, WAVE_ERR_VOLUME = 3u };
 // dbg words: queue length, fetch counter, busy ballot, exhausted, then for
 // the warp's first busy lane: ray index, origin xyz, tmax, direction xyz,
-// stack depth, group base, group hits, group internal mask, steps of the ray.
-constexpr uint32_t WAVE_DBG_WORDS = 24;
+// stack depth, group base, group hits, group internal mask; the warp's trips
+// and active mask.
+constexpr uint32_t WAVE_DBG_WORDS = 18;
 // Counter words after the per-wave block: wave, error, 2 spare, dbg.
 inline size_t wave_counter_alloc_bytes(int max_iter) { return (wave_counter_words(max_iter) + 4 + WAVE_DBG_WORDS) * 4; }
 
