@@ -14,6 +14,7 @@
 #include "scene_build.h"
 #include "traverse.cuh"
 #include "tuning.h"
+#include "warp_feed.cuh"
 
 using namespace phc;
 
@@ -43,29 +44,27 @@ int fail(int code, const std::string &m)
   return code;
 }
 
-constexpr uint32_t FULL = 0xffffffffu;
-
-// One ray per thread; persistent warps take 32-ray batches.  INST: the
-// accel holds instances (two-level traversal); full hit records then follow
-// the reference's instanced back-end (photon_optix.cu:68-99, 161-187): the
+// One ray per thread.  SHORT: a call of at most one batch of rays per warp gives
+// every warp its place in the grid, with fewer than 32 rays each when there
+// are not enough for half of the warps (spread_lanes), and reads no counter;
+// longer calls have persistent warps that take 32-ray batches from `fetch`.
+// 1,000 rays against a 6,000-triangle mesh 54 -> 43 us a call, 30,000 bounce
+// rays 93 -> 80 us; long calls keep their own kernel because the shared one cost
+// them 2% (its batch size and last batch in registers).  Refilling idle lanes
+// as k_trace does was measured and dropped: 723K bounce rays 459 -> 421 us, but
+// 1M camera rays 315 -> 366 us (12% more instructions, and nothing to win where
+// neighbouring rays end together).
+// INST: the accel holds instances (two-level traversal); full hit records then
+// follow the reference's instanced back-end (photon_optix.cu:68-99, 161-187): the
 // barycentrics as uv, the primitive's index within its object, the object's
 // index as inst_id (the object count for the accel's own triangles).
-template <int MODE, bool COUNT, bool INST = false> // MODE 0 full hit record, 1 compact, 2 occluded
+template <int MODE, bool SHORT, bool COUNT, bool INST = false> // MODE 0 full hit record, 1 compact, 2 occluded
 __global__ void __launch_bounds__(128) k_level_a(DevScene sc, const float *__restrict__ orgs,
     const float *__restrict__ dirs, const float *__restrict__ tmins, const float *__restrict__ tmaxs, uint32_t n,
     void *out, uint32_t *fetch, unsigned long long *stats)
 {
   TravCounters ctr{0u, 0u};
-  for (;;) {
-    uint32_t base = 0;
-    if ((threadIdx.x & 31u) == 0)
-      base = atomicAdd(fetch, 32u);
-    base = __shfl_sync(FULL, base, 0);
-    if (base >= n)
-      break;
-    const uint32_t i = base + (threadIdx.x & 31u);
-    if (i >= n)
-      continue;
+  auto trace = [&](uint32_t i) {
     const size_t i3 = size_t(3) * i;
     const V3 o{orgs[i3], orgs[i3 + 1], orgs[i3 + 2]};
     const V3 d{dirs[i3], dirs[i3 + 1], dirs[i3 + 2]};
@@ -75,13 +74,13 @@ __global__ void __launch_bounds__(128) k_level_a(DevScene sc, const float *__res
       const RayHit h = INST ? trace_ray2<true, COUNT>(sc, o, d, t0, t1, &ctr, inst)
                             : trace_ray<true, COUNT>(sc, o, d, t0, t1, &ctr);
       static_cast<uint32_t *>(out)[i] = h.prim != 0xffffffffu ? 1u : 0u;
-      continue;
+      return;
     }
     const RayHit h = INST ? trace_ray2<false, COUNT>(sc, o, d, t0, t1, &ctr, inst)
                           : trace_ray<false, COUNT>(sc, o, d, t0, t1, &ctr);
     if (MODE == 1) {
       reinterpret_cast<float4 *>(out)[i] = make_float4(h.t, __uint_as_float(h.prim), h.u, h.v);
-      continue;
+      return;
     }
     // HitResult (ray_backend.h:15-29); like KokkosBackend only `hit` is written
     // for a miss, here the record is zeroed instead.
@@ -121,11 +120,48 @@ __global__ void __launch_bounds__(128) k_level_a(DevScene sc, const float *__res
     float *dst = static_cast<float *>(out) + size_t(i) * 22;
     for (int k = 0; k < 22; ++k)
       dst[k] = rec[k];
+  };
+  if (SHORT) {
+    const uint32_t per_warp = spread_lanes(n);
+    const uint32_t i = (blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5)) * per_warp + lane_id();
+    if (lane_id() < per_warp && i < n)
+      trace(i);
+  } else {
+    for (;;) {
+      const uint32_t base = warp_fetch(fetch);
+      if (base >= n)
+        break;
+      if (base + lane_id() < n)
+        trace(base + lane_id());
+    }
   }
   if (COUNT) {
     atomicAdd(&stats[0], (unsigned long long)ctr.nodes);
     atomicAdd(&stats[1], (unsigned long long)ctr.tris);
   }
+}
+
+constexpr int LEVEL_A_BLOCKS = 16; // per SM, of 128 threads
+
+// Whether n rays are at most one batch per warp (and need no batch counter).
+bool level_a_short(const phc_accel *a, uint32_t n) { return n <= uint32_t(a->sm_count * LEVEL_A_BLOCKS) * 4u * 32u; }
+
+// The traversal of n > 0 rays on stream s; a long call's counter `fetch` is 0.
+template <int MODE, bool COUNT>
+void launch_level_a(const phc_accel *a, const float *o, const float *d, const float *t0, const float *t1, uint32_t n,
+    void *out, uint32_t *fetch, unsigned long long *stats, cudaStream_t s)
+{
+  const DevScene &sc = a->scene.dev;
+  const int blocks = a->sm_count * LEVEL_A_BLOCKS;
+  const bool brief = level_a_short(a, n), inst = sc.inst_count > 0;
+  if (brief && inst)
+    k_level_a<MODE, true, COUNT, true><<<blocks, 128, 0, s>>>(sc, o, d, t0, t1, n, out, fetch, stats);
+  else if (brief)
+    k_level_a<MODE, true, COUNT><<<blocks, 128, 0, s>>>(sc, o, d, t0, t1, n, out, fetch, stats);
+  else if (inst)
+    k_level_a<MODE, false, COUNT, true><<<blocks, 128, 0, s>>>(sc, o, d, t0, t1, n, out, fetch, stats);
+  else
+    k_level_a<MODE, false, COUNT><<<blocks, 128, 0, s>>>(sc, o, d, t0, t1, n, out, fetch, stats);
 }
 
 template <int MODE>
@@ -148,21 +184,16 @@ int launch(phc_accel *a, const float *o, const float *d, const float *t0, const 
     return fail(PHC_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : a->stream;
   uint32_t *fetch = reinterpret_cast<uint32_t *>(a->counters + 2);
-  e = cudaMemsetAsync(a->counters, 0, 4 * sizeof(uint64_t), s);
+  const bool count = tuning().count_traversal != 0;
+  if (count || !level_a_short(a, n))
+    e = cudaMemsetAsync(a->counters, 0, 4 * sizeof(uint64_t), s);
   if (e != cudaSuccess)
     return fail(PHC_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-  const int blocks = a->sm_count * 16;
-  const bool count = tuning().count_traversal != 0;
   auto *st = reinterpret_cast<unsigned long long *>(a->counters);
-  const bool inst = a->scene.dev.inst_count > 0;
-  if (count && inst)
-    k_level_a<MODE, true, true><<<blocks, 128, 0, s>>>(a->scene.dev, o, d, t0, t1, n, out, fetch, st);
-  else if (count)
-    k_level_a<MODE, true><<<blocks, 128, 0, s>>>(a->scene.dev, o, d, t0, t1, n, out, fetch, st);
-  else if (inst)
-    k_level_a<MODE, false, true><<<blocks, 128, 0, s>>>(a->scene.dev, o, d, t0, t1, n, out, fetch, st);
+  if (count)
+    launch_level_a<MODE, true>(a, o, d, t0, t1, n, out, fetch, st, s);
   else
-    k_level_a<MODE, false><<<blocks, 128, 0, s>>>(a->scene.dev, o, d, t0, t1, n, out, fetch, st);
+    launch_level_a<MODE, false>(a, o, d, t0, t1, n, out, fetch, st, s);
   e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(s);
@@ -415,15 +446,11 @@ extern "C" int phc_trace_closest_compact_static(phc_accel *a, const float *origi
     return fail(PHC_ERR_CUDA, err);
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : a->stream;
   // the batch counter must start at zero; the array keeps the last call's value
-  e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t), s);
+  if (!level_a_short(a, n))
+    e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess)
     return fail(PHC_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-  if (a->scene.dev.inst_count)
-    k_level_a<1, false, true><<<a->sm_count * 16, 128, 0, s>>>(a->scene.dev, origins, directions, tmin, tmax, n,
-        hits4, scratch, nullptr);
-  else
-    k_level_a<1, false><<<a->sm_count * 16, 128, 0, s>>>(a->scene.dev, origins, directions, tmin, tmax, n, hits4,
-        scratch, nullptr);
+  launch_level_a<1, false>(a, origins, directions, tmin, tmax, n, hits4, scratch, nullptr, s);
   e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(s);
