@@ -23,12 +23,10 @@ struct phc_accel {
   int sm_count{0};
   cudaStream_t stream{nullptr};
   DeviceScene scene;
-  uint64_t *counters{nullptr};
+  uint64_t *counters{nullptr}; // node visits, triangle tests, batch counter (the scene's aux memory)
   uint64_t last_nodes{0}, last_tris{0};
   ~phc_accel()
   {
-    if (counters)
-      cudaFree(counters);
     if (stream)
       cudaStreamDestroy(stream);
   }
@@ -242,8 +240,6 @@ int phc_accel_create_instanced(phc_accel **out, const float *positions, uint64_t
     cudaGetDevice(&a->device);
     cudaDeviceGetAttribute(&a->sm_count, cudaDevAttrMultiProcessorCount, a->device);
     cudaError_t e = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess)
-      e = cudaMalloc(&a->counters, 4 * sizeof(uint64_t));
     if (e != cudaSuccess) {
       delete a;
       return fail(PHC_ERR_CUDA, std::string("accel: ") + cudaGetErrorString(e));
@@ -283,6 +279,8 @@ int phc_accel_create_instanced(phc_accel **out, const float *positions, uint64_t
       delete a;
       return fail(PHC_ERR_CUDA, err);
     }
+    static_assert(DeviceScene::AUX_BYTES >= 4 * sizeof(uint64_t), "accel counters");
+    a->counters = static_cast<uint64_t *>(a->scene.aux);
     if (a->scene.bvh_depth >= 64) {
       delete a;
       return fail(PHC_ERR_LIMIT, "BVH deeper than the traversal stack (64 levels)");

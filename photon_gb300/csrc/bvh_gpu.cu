@@ -1045,6 +1045,21 @@ __global__ void __launch_bounds__(256) k_leaf_records(Collapse c, const int *__r
   }
 }
 
+// The triangle records by primitive, for shading (build_prim_records of the
+// host build).
+__global__ void __launch_bounds__(256) k_prim_records(const float4 *__restrict__ pos, const uint4 *__restrict__ vidx,
+    uint32_t n, float4 *__restrict__ geo)
+{
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint4 vi = vidx[i];
+    const float4 v0 = pos[vi.x], v1 = pos[vi.y], v2 = pos[vi.z];
+    float4 *r = geo + 3 * size_t(i);
+    r[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(i));
+    r[1] = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.f);
+    r[2] = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.f);
+  }
+}
+
 // counters: [0] nodes, [1] triangle records, [3] error, [4..6] lengths of the
 // level's, the next and the one after's queue, in turn ([4] starts at 1, the
 // root's entry in q0), [7] levels.  Every block reads the same length after a
@@ -1200,9 +1215,10 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
   }
   // a BVH8 over n leaves with >= 2 children per inner node has fewer nodes
   sc.want(nodes_big, size_t(n) * 20);
+  float4 *tris_big = nullptr; // the greedy collapse writes its records as it goes
+  if (!program)
+    sc.want(tris_big, size_t(n) * 3);
   sc.allocate();
-  DevBuf tris_buf; // owned here until the build succeeds
-  alloc(tris_buf, size_t(n) * 48, "bvh8 triangles");
   // scene centroid bounds start at (+max, -max) in the ordered encoding
   const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   ck(cudaMemcpyAsync(cb, init, sizeof(init), cudaMemcpyHostToDevice, s), "bounds init");
@@ -1246,7 +1262,7 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
   ck(cudaMemcpyAsync(ctr, c0, sizeof(c0), cudaMemcpyHostToDevice, s), "collapse counters");
   const uint2 first = make_uint2(0u, result[1]);
   ck(cudaMemcpyAsync(q[0], &first, sizeof(first), cudaMemcpyHostToDevice, s), "first queue entry");
-  Collapse col{nbox, nchild, positions, prim_vidx, nodes_big, tris_buf.as<float4>(), ctr, n, leaf_max};
+  Collapse col{nbox, nchild, positions, prim_vidx, nodes_big, tris_big, ctr, n, leaf_max};
   uint32_t cc[8];
   auto read_counters = [&](const char *what) {
     ck(cudaMemcpyAsync(cc, ctr, sizeof(cc), cudaMemcpyDeviceToHost, s), "read collapse counters");
@@ -1265,8 +1281,6 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
     const uint32_t blocks = std::min<uint32_t>(most, (n + COLLAPSE_BLOCK / 8 - 1) / (COLLAPSE_BLOCK / 8));
     ck(cudaLaunchCooperativeKernel((const void *)k_collapse_sah, dim3(blocks), dim3(COLLAPSE_BLOCK), args, 0, s),
         "collapse launch");
-    k_leaf_records<<<(n + 255) / 256, 256, 0, s>>>(col, leaf_node, n);
-    ck(cudaGetLastError(), "leaf records launch");
     read_counters("collapse");
     if (cc[7] >= COLLAPSE_LEVELS)
       throw std::runtime_error("gpu bvh build: collapse did not end");
@@ -1290,13 +1304,27 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
   out.tri_count = cc[1];
   if (out.tri_count != n)
     throw std::runtime_error("gpu bvh build: leaf records do not cover the triangles");
-  DevBuf exact; // the nodes made, out of the worst-case array
-  alloc(exact, size_t(out.node_count) * 80, "bvh8 nodes");
-  ck(cudaMemcpyAsync(exact.p, nodes_big, size_t(out.node_count) * 80, cudaMemcpyDeviceToDevice, s), "nodes");
-  ck(cudaStreamSynchronize(s), "bvh8 build");
-  out.nodes = exact.p;
-  out.tris = tris_buf.p;
-  exact.p = tris_buf.p = nullptr; // ownership passes to the caller
+  // what the scene keeps, in one allocation: the nodes made (out of the
+  // worst-case array) and the triangle records in leaf and in primitive order
+  DevBuf keep; // owned here until the build succeeds
+  const size_t node_bytes = (size_t(out.node_count) * 80 + 255) & ~size_t(255);
+  out.bytes = node_bytes + size_t(n) * 96;
+  alloc(keep, out.bytes, "bvh8");
+  out.nodes = keep.p;
+  out.tris = keep.as<char>() + node_bytes;
+  out.geo = keep.as<char>() + node_bytes + size_t(n) * 48;
+  ck(cudaMemcpyAsync(out.nodes, nodes_big, size_t(out.node_count) * 80, cudaMemcpyDeviceToDevice, s), "nodes");
+  if (program) {
+    col.tris = static_cast<float4 *>(out.tris);
+    k_leaf_records<<<(n + 255) / 256, 256, 0, s>>>(col, leaf_node, n);
+    ck(cudaGetLastError(), "leaf records launch");
+  } else {
+    ck(cudaMemcpyAsync(out.tris, tris_big, size_t(n) * 48, cudaMemcpyDeviceToDevice, s), "triangles");
+  }
+  k_prim_records<<<grid_of(n, 256), 256, 0, s>>>(positions, prim_vidx, n, static_cast<float4 *>(out.geo));
+  ck(cudaGetLastError(), "primitive records launch");
+  read_counters("bvh8 build"); // (the leaf records check their sizes)
+  keep.p = nullptr; // ownership passes to the caller
   return out;
 }
 

@@ -10,8 +10,10 @@
 namespace phc {
 
 struct GpuBvh8 {
-  void *nodes{nullptr}; // node_cap x 80 bytes (cudaMalloc; the caller frees)
-  void *tris{nullptr};  // tri_count x 48 bytes (cudaMalloc; the caller frees)
+  void *nodes{nullptr}; // node_cap x 80 bytes (cudaMalloc; the caller frees it, and with it the others)
+  void *tris{nullptr};  // tri_count x 48 bytes, in the same allocation
+  void *geo{nullptr};   // the same records by primitive (DevScene::prim_geo), likewise
+  size_t bytes{0};      // of the allocation
   uint32_t node_count{0}, node_cap{0}, tri_count{0}, max_depth{0};
 };
 

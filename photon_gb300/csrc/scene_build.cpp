@@ -14,6 +14,7 @@
 #include <cstring>
 #include <limits>
 #include <stdexcept>
+#include <omp.h>
 
 namespace phc {
 namespace {
@@ -680,67 +681,77 @@ void build_host_scene(const phc_scene_desc &in, HostScene &s)
   }
   if (tc > 0x3fffffffull || vc > 0xffffffffull)
     throw std::length_error("scene: too many triangles or vertices");
-  // the per-vertex and per-triangle arrays, each filled by one parallel loop
-  // (element by element the same values as a sequential copy)
-  HostVec<float> pos3(vc * 3);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < int64_t(vc * 3); ++i)
-    pos3[size_t(i)] = empty ? 0.f : in.positions[i];
-  // the scene's extent, in vertex order (RenderBridge.cpp:815-820)
-  float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
-  for (size_t i = 0; i < vc; ++i)
-    for (int a = 0; a < 3; ++a) {
-      const float p = pos3[3 * i + a];
-      lo[a] = lo[a] < p ? lo[a] : p;
-      hi[a] = hi[a] > p ? hi[a] : p;
-    }
-  s.indices.resize(tc * 3);
-  int bad_index = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad_index)
-  for (int64_t i = 0; i < int64_t(tc * 3); ++i) {
-    const uint32_t v = empty ? uint32_t(i) : in.indices[i];
-    bad_index |= v >= vc ? 1 : 0;
-    s.indices[size_t(i)] = v;
-  }
-  if (bad_index)
-    throw std::out_of_range("scene: vertex index out of range");
-  const uint32_t material_count = uint32_t(std::max<size_t>(in.material_count, 1));
-  s.material_ids.resize(tc);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < int64_t(tc); ++i) {
-    const uint32_t id =
-        (!empty && in.material_ids && uint64_t(i) < in.material_id_count) ? in.material_ids[i] : 0u;
-    s.material_ids[size_t(i)] = id < material_count ? id : 0u;
-  }
-  s.positions4.resize(vc * 4);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < int64_t(vc); ++i) {
-    s.positions4[4 * size_t(i)] = pos3[3 * size_t(i)];
-    s.positions4[4 * size_t(i) + 1] = pos3[3 * size_t(i) + 1];
-    s.positions4[4 * size_t(i) + 2] = pos3[3 * size_t(i) + 2];
-    s.positions4[4 * size_t(i) + 3] = 0.f;
-  }
-  if (!empty && in.normals) {
-    s.normals4.resize(vc * 4);
-#pragma omp parallel for schedule(static)
-    for (int64_t i = 0; i < int64_t(vc); ++i) {
-      s.normals4[4 * size_t(i)] = in.normals[3 * i];
-      s.normals4[4 * size_t(i) + 1] = in.normals[3 * i + 1];
-      s.normals4[4 * size_t(i) + 2] = in.normals[3 * i + 2];
-      s.normals4[4 * size_t(i) + 3] = 0.f;
-    }
-  }
-  s.prim_vidx.resize(tc * 4);
-#pragma omp parallel for schedule(static)
-  for (int64_t t = 0; t < int64_t(tc); ++t) {
-    s.prim_vidx[4 * size_t(t)] = s.indices[3 * size_t(t)];
-    s.prim_vidx[4 * size_t(t) + 1] = s.indices[3 * size_t(t) + 1];
-    s.prim_vidx[4 * size_t(t) + 2] = s.indices[3 * size_t(t) + 2];
-    s.prim_vidx[4 * size_t(t) + 3] = s.material_ids[size_t(t)];
-  }
-  s.prim_geo.resize(tc * 12);
-  build_prim_records(pos3.data(), s.indices.data(), tc, s.prim_geo.data());
   const phc_pt_scene *pt = in.pt;
+  const bool instanced = pt && pt->instance_count && pt->object_count;
+  s.bvh_on_gpu = tuning().gpu_bvh && !instanced && !empty; // single-level scenes: the upload builds the BVH8
+  static const float no_positions[9] = {};
+  const float *pos3 = empty ? no_positions : in.positions;
+  const uint32_t material_count = uint32_t(std::max<size_t>(in.material_count, 1));
+  const bool normals = !empty && in.normals;
+  s.positions4.resize(vc * 4);
+  s.normals4.resize(normals ? vc * 4 : 0);
+  s.material_ids.resize(tc);
+  s.prim_vidx.resize(tc * 4);
+  if (!s.bvh_on_gpu)
+    s.indices.resize(tc * 3);
+  // The per-vertex and per-triangle arrays, filled by one parallel region (on
+  // one core when they are small: waking the others costs 23 us), each thread a
+  // run of consecutive elements, and the scene's extent in vertex order
+  // (RenderBridge.cpp:815-820): lo < p ? lo : p takes p where lo is NaN, so a
+  // run that holds a NaN forgets what was before it.
+  struct Run {
+    float lo[3], hi[3];
+    bool nan[3];
+    bool any, bad_index;
+  };
+  std::vector<Run> runs(size_t(std::max(omp_get_max_threads(), 1)));
+#pragma omp parallel if (vc + tc > 16384)
+  {
+    const size_t t = size_t(omp_get_thread_num()), of = size_t(omp_get_num_threads());
+    Run r{};
+    for (size_t i = vc * t / of; i < vc * (t + 1) / of; ++i) {
+      for (int a = 0; a < 3; ++a) {
+        const float p = pos3[3 * i + a];
+        s.positions4[4 * i + a] = p;
+        r.nan[a] = r.nan[a] || p != p;
+        r.lo[a] = r.any && r.lo[a] < p ? r.lo[a] : p;
+        r.hi[a] = r.any && r.hi[a] > p ? r.hi[a] : p;
+      }
+      r.any = true;
+      s.positions4[4 * i + 3] = 0.f;
+      if (normals) {
+        for (int a = 0; a < 3; ++a)
+          s.normals4[4 * i + a] = in.normals[3 * i + a];
+        s.normals4[4 * i + 3] = 0.f;
+      }
+    }
+    for (size_t i = tc * t / of; i < tc * (t + 1) / of; ++i) {
+      const uint32_t id = !empty && in.material_ids && i < in.material_id_count ? in.material_ids[i] : 0u;
+      s.material_ids[i] = id < material_count ? id : 0u;
+      for (int k = 0; k < 3; ++k) {
+        const uint32_t v = empty ? uint32_t(3 * i + k) : in.indices[3 * i + k];
+        r.bad_index = r.bad_index || v >= vc;
+        s.prim_vidx[4 * i + k] = v;
+        if (!s.bvh_on_gpu)
+          s.indices[3 * i + k] = v;
+      }
+      s.prim_vidx[4 * i + 3] = s.material_ids[i];
+    }
+    runs[t] = r;
+  }
+  float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
+  for (const Run &r : runs) {
+    if (r.bad_index)
+      throw std::out_of_range("scene: vertex index out of range");
+    for (int a = 0; r.any && a < 3; ++a) {
+      lo[a] = !r.nan[a] && lo[a] < r.lo[a] ? lo[a] : r.lo[a];
+      hi[a] = !r.nan[a] && hi[a] > r.hi[a] ? hi[a] : r.hi[a];
+    }
+  }
+  if (!s.bvh_on_gpu) {
+    s.prim_geo.resize(tc * 12);
+    build_prim_records(pos3, s.indices.data(), tc, s.prim_geo.data());
+  }
   if (pt) {
     if (in.material_count && !pt->materials)
       throw std::invalid_argument("scene: pt materials pointer is null");
@@ -909,15 +920,17 @@ void build_host_scene(const phc_scene_desc &in, HostScene &s)
   // and area densities (pathtracer.cpp:439-487)
   std::vector<uint32_t> ids;
   std::vector<float> areas;
-  const bool instanced = pt && pt->instance_count && pt->object_count;
-  s.emissive_on_gpu = !empty && !instanced && tuning().gpu_tables; // built by the upload
-  if (!empty && !s.emissive_on_gpu) {
+  bool emitters = false; // without a material that may emit there is nothing to look for
+  for (const DevMaterial &m : s.materials)
+    emitters = emitters || tbl_may_emit(m);
+  s.emissive_on_gpu = !empty && !instanced && emitters && tuning().gpu_tables; // built by the upload
+  if (!empty && emitters && !s.emissive_on_gpu) {
     for (size_t t = 0; t < tc; ++t) {
       const uint32_t mid = s.material_ids[t];
       if (!tbl_may_emit(s.materials[mid]))
         continue;
-      const float area = tbl_tri_area(&pos3[3 * size_t(s.indices[3 * t])], &pos3[3 * size_t(s.indices[3 * t + 1])],
-          &pos3[3 * size_t(s.indices[3 * t + 2])]);
+      const float area = tbl_tri_area(&pos3[3 * size_t(s.prim_vidx[4 * t])], &pos3[3 * size_t(s.prim_vidx[4 * t + 1])],
+          &pos3[3 * size_t(s.prim_vidx[4 * t + 2])]);
       if (!(area > 0.f))
         continue;
       ids.push_back(uint32_t(t));
@@ -956,11 +969,9 @@ void build_host_scene(const phc_scene_desc &in, HostScene &s)
   s.strategy_count = uint32_t(s.lights.size()) + (s.emissive_cdf.empty() ? 0u : 1u) + (s.has_env ? 1u : 0u);
   build_search_guides(s);
   s.scene_normals = !empty && in.normals;
-  if (tuning().gpu_bvh && !instanced && !empty) {
-    s.bvh_on_gpu = true; // single-level scenes: the upload builds the BVH8 on the GPU
+  if (s.bvh_on_gpu)
     return;
-  }
-  build_bvh8(pos3.data(), vc, s.indices.data(), tc, s.bvh, tuning().max_leaf);
+  build_bvh8(pos3, vc, s.indices.data(), tc, s.bvh, tuning().max_leaf);
   if (instanced)
     build_instancing(*pt, !empty, lo, hi, s, tuning().max_leaf);
 }
@@ -976,22 +987,71 @@ void DeviceScene::release()
   allocations.clear();
   dev = DevScene{};
   bytes = 0;
+  arena = nullptr;
+  arena_used = arena_size = 0;
+  aux = nullptr;
 }
 
-template <class T, class A> T *DeviceScene::put(const std::vector<T, A> &v, cudaStream_t s, std::string &err)
+// n bytes of the scene's memory: from the arena, or an allocation of their own.
+void *DeviceScene::take(size_t n, std::string &err)
 {
-  if (v.empty() || !err.empty())
-    return nullptr;
+  const size_t padded = (n + 255) & ~size_t(255);
+  if (padded <= arena_size - arena_used) {
+    void *p = arena + arena_used;
+    arena_used += padded;
+    bytes += n;
+    return p;
+  }
   void *p = nullptr;
-  const size_t n = v.size() * sizeof(T);
-  cudaError_t e = cudaMalloc(&p, n);
+  const cudaError_t e = cudaMalloc(&p, n);
   if (e != cudaSuccess) {
     err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return nullptr;
   }
   allocations.push_back(p);
   bytes += n;
-  e = cudaMemcpyAsync(p, v.data(), n, cudaMemcpyHostToDevice, s);
+  return p;
+}
+
+// The arena's size: the arrays whose sizes are known before the upload.
+size_t DeviceScene::arena_bytes(const HostScene &h) const
+{
+  size_t n = 0;
+  auto add = [&](size_t b) { n += (b + 255) & ~size_t(255); };
+  auto vec = [&](const auto &v) { add(v.size() * sizeof(v[0])); };
+  add(AUX_BYTES);
+  vec(h.bvh.nodes), vec(h.bvh.tris), vec(h.prim_geo), vec(h.prim_vidx), vec(h.normals4), vec(h.positions4);
+  vec(h.materials), vec(h.attr_values), vec(h.u8_decode), vec(h.texels_u8), vec(h.samplers), vec(h.lights);
+  vec(h.emissive_ids), vec(h.emissive_cdf), vec(h.prim_light_pdf), vec(h.env_pixels4), vec(h.env_marginal);
+  vec(h.env_conditional), vec(h.emissive_guide), vec(h.env_mguide), vec(h.env_cguide), vec(h.volumes);
+  vec(h.vol_tf), vec(h.vol_majorants), vec(h.inst_w2o), vec(h.inst_info);
+  size_t texels = h.texels.size(), values = h.vol_values.size();
+  for (const HostScene::Span &sp : h.texel_spans)
+    texels += sp.floats;
+  for (const HostScene::Span &sp : h.vol_value_spans)
+    values += sp.floats;
+  add(texels * 4), add(values * 4), add(h.texels_u8_device * 4);
+  if (h.env_rgb) { // device_tables
+    const size_t w = h.env_w, eh = h.env_h;
+    add(w * eh * 16), add(eh * (w + 1) * 4), add((eh + 1) * 4);
+    add(((size_t(1) << ENV_MGUIDE_BITS) + 1) * 4), add(eh * ((size_t(1) << ENV_CGUIDE_BITS) + 1) * 4);
+  }
+  if (h.emissive_on_gpu) { // the densities, and the ids and CDF of up to 4096 emitters
+    add(h.prim_vidx.size()), add(((size_t(1) << EMISSIVE_GUIDE_BITS) + 1) * 4);
+    add(4096 * 4), add(4096 * 4);
+  }
+  return n;
+}
+
+template <class T, class A> T *DeviceScene::put(const std::vector<T, A> &v, cudaStream_t s, std::string &err)
+{
+  if (v.empty() || !err.empty())
+    return nullptr;
+  const size_t n = v.size() * sizeof(T);
+  void *p = take(n, err);
+  if (!p)
+    return nullptr;
+  const cudaError_t e = cudaMemcpyAsync(p, v.data(), n, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess)
     err = std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e);
   return static_cast<T *>(p);
@@ -1008,15 +1068,10 @@ float *DeviceScene::put_spans(const std::vector<float> &owned, const std::vector
     total += sp.floats;
   if (total == 0 || !err.empty())
     return nullptr;
-  void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, total * sizeof(float));
-  if (e != cudaSuccess) {
-    err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+  cudaError_t e = cudaSuccess;
+  float *dst = static_cast<float *>(take(total * sizeof(float), err));
+  if (!dst)
     return nullptr;
-  }
-  allocations.push_back(p);
-  bytes += total * sizeof(float);
-  float *dst = static_cast<float *>(p);
   if (!owned.empty())
     e = cudaMemcpyAsync(dst, owned.data(), owned.size() * sizeof(float), cudaMemcpyHostToDevice, s);
   size_t at = owned.size();
@@ -1030,21 +1085,9 @@ float *DeviceScene::put_spans(const std::vector<float> &owned, const std::vector
   return dst;
 }
 
-template <class T> T *DeviceScene::alloc(size_t n, std::string &err, bool keep)
+template <class T> T *DeviceScene::alloc(size_t n, std::string &err)
 {
-  if (!err.empty() || n == 0)
-    return nullptr;
-  void *p = nullptr;
-  const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) {
-    err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-    return nullptr;
-  }
-  if (keep) {
-    allocations.push_back(p);
-    bytes += n * sizeof(T);
-  }
-  return static_cast<T *>(p);
+  return err.empty() && n ? static_cast<T *>(take(n * sizeof(T), err)) : nullptr;
 }
 
 // The environment and emitter tables of h built on the device
@@ -1057,12 +1100,33 @@ template <class T> T *DeviceScene::alloc(size_t n, std::string &err, bool keep)
 std::string DeviceScene::device_tables(const HostScene &h, DevScene &d, cudaStream_t s)
 {
   std::string err;
+  // the call's scratch: one allocation for what is known beforehand
+  const uint32_t tri_count = uint32_t(h.prim_vidx.size() / 4);
+  const size_t env_texels = h.env_rgb ? size_t(h.env_w) * h.env_h : 0, tri_scratch = h.emissive_on_gpu ? tri_count : 0;
+  const size_t scratch_size = 256 * 8 + env_texels * 12 + size_t(h.env_rgb ? h.env_h : 0) * 8 +
+      (2 * tri_scratch + scan_u32_scratch(uint32_t(tri_scratch))) * 4;
+  char *scratch_arena = nullptr;
+  size_t scratch_used = 0;
   std::vector<void *> scratch;
-  auto tmp = [&](size_t bytes_) -> void * {
-    void *p = alloc<uint8_t>(bytes_, err, false);
-    if (p)
+  {
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&scratch_arena), scratch_size);
+    if (e != cudaSuccess)
+      return std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    scratch.push_back(scratch_arena);
+  }
+  auto tmp = [&](size_t n) -> void * {
+    const size_t padded = (n + 255) & ~size_t(255);
+    if (padded <= scratch_size - scratch_used) {
+      scratch_used += padded;
+      return scratch_arena + scratch_used - padded;
+    }
+    void *p = nullptr;
+    const cudaError_t e = err.empty() ? cudaMalloc(&p, n) : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess)
       scratch.push_back(p);
-    return p;
+    else if (err.empty())
+      err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    return e == cudaSuccess ? p : nullptr;
   };
   auto ck = [&](cudaError_t e, const char *what) {
     if (e != cudaSuccess && err.empty())
@@ -1105,7 +1169,7 @@ std::string DeviceScene::device_tables(const HostScene &h, DevScene &d, cudaStre
   }
   EmissiveJob ej{};
   uint32_t counts[4] = {0, 0, 0, 0};
-  const uint32_t tc = uint32_t(h.prim_vidx.size() / 4);
+  const uint32_t tc = tri_count;
   if (h.emissive_on_gpu && err.empty() && tc) {
     ej.pos = d.positions;
     ej.vidx = d.prim_vidx;
@@ -1197,12 +1261,10 @@ const uchar4 *DeviceScene::pack_texels(const HostScene &h, std::vector<DevSample
   for (const HostScene::TexelPackTask &t : h.texel_pack_tasks)
     most = std::max(most, t.texels);
   void *out = nullptr, *stage = nullptr, *bad = nullptr;
-  cudaError_t e = cudaMalloc(&out, h.texels_u8_device * sizeof(uchar4));
-  if (e == cudaSuccess) {
-    allocations.push_back(out);
-    bytes += h.texels_u8_device * sizeof(uchar4);
-    e = cudaMalloc(&bad, n_tasks * sizeof(uint32_t));
-  }
+  out = take(h.texels_u8_device * sizeof(uchar4), err);
+  if (!out)
+    return nullptr;
+  cudaError_t e = cudaMalloc(&bad, n_tasks * sizeof(uint32_t));
   if (e == cudaSuccess)
     e = cudaMemsetAsync(bad, 0, n_tasks * sizeof(uint32_t), s);
   uchar4 *dst = static_cast<uchar4 *>(out);
@@ -1253,6 +1315,15 @@ std::string DeviceScene::upload(const HostScene &h, cudaStream_t s)
   release();
   std::string err;
   DevScene d{};
+  const size_t known = arena_bytes(h);
+  arena = static_cast<char *>(take(known, err));
+  if (!arena) {
+    release();
+    return err;
+  }
+  arena_size = known;
+  bytes = 0; // counted as the arrays are taken
+  aux = take(AUX_BYTES, err);
   d.nodes = reinterpret_cast<const uint4 *>(put(h.bvh.nodes, s, err));
   d.tris = reinterpret_cast<const float4 *>(put(h.bvh.tris, s, err));
   d.prim_geo = reinterpret_cast<const float4 *>(put(h.prim_geo, s, err));
@@ -1348,11 +1419,11 @@ std::string DeviceScene::upload(const HostScene &h, cudaStream_t s)
     try {
       const GpuBvh8 g = build_bvh8_gpu(d.positions, d.prim_vidx, uint32_t(h.prim_vidx.size() / 4), s,
           tuning().gpu_max_leaf, tuning().ploc_radius, 0.01f * float(tuning().collapse_tri_cost));
-      allocations.push_back(g.nodes);
-      allocations.push_back(g.tris);
-      bytes += size_t(g.node_cap) * 80 + size_t(g.tri_count) * 48;
+      allocations.push_back(g.nodes); // the records lie in its allocation
+      bytes += g.bytes;
       d.nodes = static_cast<const uint4 *>(g.nodes);
       d.tris = static_cast<const float4 *>(g.tris);
+      d.prim_geo = static_cast<const float4 *>(g.geo);
       d.node_count = g.node_count;
       node_bytes = uint64_t(g.node_count) * 80;
       tri_bytes = uint64_t(g.tri_count) * 48;

@@ -48,7 +48,7 @@ struct HostScene {
   HostVec<uint32_t> material_ids; // clamped like the bridge
   HostVec<float> normals4;        // empty: none
   HostVec<uint32_t> prim_vidx;    // (i0, i1, i2, material) per triangle
-  HostVec<float> prim_geo;        // 12 floats per triangle
+  HostVec<float> prim_geo;        // 12 floats per triangle (empty with bvh_on_gpu: made there)
   std::vector<DevMaterial> materials;
   std::vector<float> attr_values;     // float4
   int32_t attr_offset[5]{-1, -1, -1, -1, -1};
@@ -133,17 +133,26 @@ struct DeviceScene {
   bool may_pass{true};           // a path may go through a surface without a bounce (scene_may_pass)
   uint32_t bvh_depth{0};
   uint64_t table_floats[5]{}; // lengths of the tables phc_scene_table reads (PHC_TABLE_*)
+  void *aux{nullptr};         // AUX_BYTES of device memory for the scene's owner
+  static constexpr size_t AUX_BYTES = 256;
   ~DeviceScene();
   void release();
   // Returns an empty string on success, else the failure message.
   std::string upload(const HostScene &h, cudaStream_t stream);
 
 private:
+  // The scene's arrays come from one allocation where they fit (arena), each
+  // from its own otherwise: an allocation and its release cost 60 us, a small
+  // scene has a dozen arrays.
+  char *arena{nullptr};
+  size_t arena_used{0}, arena_size{0};
+  void *take(size_t n, std::string &err);
+  size_t arena_bytes(const HostScene &h) const;
   template <class T, class A> T *put(const std::vector<T, A> &v, cudaStream_t s, std::string &err);
   float *put_spans(const std::vector<float> &owned, const std::vector<HostScene::Span> &spans, cudaStream_t s,
       std::string &err);
   std::string device_tables(const HostScene &h, DevScene &d, cudaStream_t s);
-  template <class T> T *alloc(size_t n, std::string &err, bool keep = true);
+  template <class T> T *alloc(size_t n, std::string &err);
   const uchar4 *pack_texels(const HostScene &h, std::vector<DevSampler> &samplers,
       std::vector<HostScene::Span> &spans, const float *dec, cudaStream_t s, std::string &err);
 };
