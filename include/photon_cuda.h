@@ -531,7 +531,8 @@ int phc_trace_closest_compact_static(phc_accel *a, const float *origins, const f
    smaller waves use one lean hit kernel),
    "shade_lean" (0/1: lean shading kernels for scenes without volumes /
    sources / lights), "sort_threshold" (sort the hit queue by material when it
-   holds at least this many hits; 0: never), "max_leaf" (1..3, leaf size of the
+   holds at least this many hits, in waves of at least 8 times as many paths;
+   0: never), "max_leaf" (1..3, leaf size of the
    host-built BVH8, read at the next scene upload), "gpu_bvh" (0/1: build
    the BVH8 of single-level scenes on the GPU, read at the next scene
    upload), "gpu_max_leaf" (1..3, leaf size of the GPU-built BVH8, read at

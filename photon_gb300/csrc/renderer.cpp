@@ -378,6 +378,12 @@ struct KernelTimer {
   }
 };
 
+// Whether a wave of this many paths sorts its hit queues at all.
+bool sorts_wave(const Tuning &tu, uint64_t wave_paths)
+{
+  return tu.sort_threshold > 0 && wave_paths >= 8 * uint64_t(tu.sort_threshold);
+}
+
 // Launches that may run beside what the main stream launches next: begin()
 // gives the stream for them, ordered after the main stream's launches so far;
 // end() marks their end, and join() makes the main stream's next launches wait
@@ -475,12 +481,22 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
   // shading code for every hit: sorting gains nothing there and the
   // shading's reads through the sorted order cost (box room 1503 against
   // 1813 Msamples/s)
-  const bool sort = split && r->scene.shade_class_count > 1 && tu.sort_threshold > 0 &&
-      wave_paths >= size_t(tu.sort_threshold);
+  // The threshold is per bounce; a wave of fewer than 8 times as many paths
+  // has so few such bounces that the sort's launches cost more than it saves
+  // (500K scene, 1024 x 1024: 1 spp 4.78 ms sorted, 4.56 unsorted; 4 spp 8.25 and
+  // 8.61).
+  const bool sort = split && r->scene.shade_class_count > 1 && sorts_wave(tu, wave_paths);
   // lean scenes: the hit queue sorted by shading class, one kernel per class
   // (waves below class_threshold paths keep one lean hit kernel: the class
-  // kernels' launches and tails cost more than they save on small waves)
+  // kernels' launches and tails cost more than they save on small waves;
+  // measured from 2^23 paths on, 500K scene: 16 spp 21.8 -> 21.4 ms, 48 spp
+  // 57.6 -> 56.1 ms)
   const bool classes = sort && !full && tu.shade_classes && wave_paths >= size_t(tu.class_threshold);
+  // else one lean hit kernel, compiled for no more lobes than the materials
+  // have between them: the box room's shading (every material diffuse) 5.43 ->
+  // 3.92 ms
+  if (split && !full && !classes && tu.shade_classes)
+    hq.whole_class = lean_class_of(r->scene.lobes);
   const size_t bin_words = size_t(2) * MAT_SORT_BINS;
   if (sort) { // sort_bins sized by ensure_wave_buffers (no allocation while a graph is captured)
     hq.sorted = r->hitq_sorted.as<uint32_t>();
@@ -545,7 +561,12 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
         launches += SHADE_CLASSES - 1;
         part_b.end();
       }
-      shade(s, 1);
+      if (hqi.whole_class) {
+        timed(2, [&] { launch_shade_class(cfg, s, rc, sc, in, out, hits, sh, ac, wc, it, hqi.whole_class, hqi); });
+        launches += 1;
+      } else {
+        shade(s, 1);
+      }
       part_a.end();
       part_a.join();
       part_b.join();
@@ -920,7 +941,7 @@ struct BatchPlan {
   std::vector<uint32_t> wave_entry, wave_items;
   uint32_t max_items{0};
   int max_iter{0};
-  uint32_t features{0};
+  uint32_t features{0}, lobes{0};
 };
 
 BatchPlan plan_batch(const std::vector<phc_renderer *> &rs, const std::vector<JobPlan> &plans, uint64_t cap)
@@ -932,6 +953,7 @@ BatchPlan plan_batch(const std::vector<phc_renderer *> &rs, const std::vector<Jo
     b.jobs.push_back(BatchJob{rs[j]->scene.dev, plans[j].rc, accum(rs[j])});
     b.max_iter = std::max(b.max_iter, plans[j].max_iter);
     b.features |= rs[j]->scene.dev.features;
+    b.lobes |= rs[j]->scene.lobes;
   }
   size_t start = 0;
   b.wave_entry.push_back(0);
@@ -965,8 +987,9 @@ BatchPlan plan_batch(const std::vector<phc_renderer *> &rs, const std::vector<Jo
   return b;
 }
 
-void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg, const BatchTable &bt, int max_iter,
-    uint32_t features, uint32_t max_items)
+// Returns the number of kernel launches.
+uint64_t record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg, const BatchTable &bt, int max_iter,
+    uint32_t features, uint32_t lobes, uint32_t max_items)
 {
   const Tuning &tu = tuning();
   const WaveCounters wc = wave_counters(lead, max_iter);
@@ -977,9 +1000,11 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
   const bool split = (features & SCENE_VOLUMES) == 0 && tu.split_shade;
   HitQueues hq =
       split ? HitQueues{lead->hitq.as<uint32_t>(), lead->missq.as<uint32_t>()} : HitQueues{nullptr, nullptr};
-  const bool sort = split && tu.sort_threshold > 0;
+  const bool sort = split && sorts_wave(tu, max_items);
   // lean batches: the hit queue sorted by shading class, one kernel per class
   const bool classes = sort && !full && tu.shade_classes && max_items >= uint64_t(tu.class_threshold);
+  if (split && !full && !classes && tu.shade_classes) // as in record_wave
+    hq.whole_class = lean_class_of(lobes);
   const size_t bin_words = size_t(2) * MAT_SORT_BINS;
   if (sort) { // sort_bins sized by ensure_wave_buffers
     hq.sorted = lead->hitq_sorted.as<uint32_t>();
@@ -988,6 +1013,7 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
     ck(cudaMemsetAsync(lead->sort_bins.p, 0, size_t(max_iter) * bin_words * 4, s), "reset sort bins");
   }
   float4 *hits = lead->hits.as<float4>();
+  uint64_t launches = 2; // ray generation, wave end
   launch_raygen_batch(cfg, s, bt, path_soa(lead, 0), wc);
   SideBranch shadows(lead, s, 0, true), part_a(lead, s, 1, true), part_b(lead, s, 2, true); // as in record_wave
   for (int it = 0; it < max_iter; ++it) {
@@ -996,6 +1022,8 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
     if (sort)
       launch_material_sort_batch(cfg, s, bt, in.info, hits, hq, wc, it,
           lead->sort_bins.as<uint32_t>() + size_t(it) * bin_words);
+    launches += 1 + (sort ? 3 : 0) + (split ? 2 : 1) + (split && classes ? SHADE_CLASSES - 1 : 0) +
+        ((features & SCENE_VOLUMES) != 0 ? 2 : 1);
     shadows.join();
     if (split) {
       HitQueues hqi = hq;
@@ -1009,7 +1037,10 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
           launch_shade_class_batch(cfg, c & 1u ? sb : s, bt, in, out, hits, sh, wc, it, c, hqi);
         part_b.end();
       }
-      launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 1}, hqi);
+      if (hqi.whole_class)
+        launch_shade_class_batch(cfg, s, bt, in, out, hits, sh, wc, it, hqi.whole_class, hqi);
+      else
+        launch_shade_batch(cfg, s, bt, in, out, hits, sh, wc, it, ShadeVariant{full, 1}, hqi);
       part_a.end();
       part_a.join();
       part_b.join();
@@ -1021,6 +1052,7 @@ void record_batch_wave(phc_renderer *lead, cudaStream_t s, const LaunchCfg &cfg,
   }
   shadows.join();
   launch_wave_end(s, nullptr, Accum{}, wc, 0, 0, max_iter, lead->stats_buf.as<uint64_t>());
+  return launches;
 }
 
 template <class T> void upload_vec(Buf &b, const std::vector<T> &v, cudaStream_t s, const char *what)
@@ -1087,12 +1119,15 @@ void render_batch_impl(const phc_job *jobs, uint32_t n, phc_render_stats *out_st
   const uint32_t waves = uint32_t(bp.wave_items.size());
   ck(cudaEventRecord(lead->ev0, s), "event");
   uint64_t launches = 0;
-  if (tu.use_graph) {
+  // one wave is launched as it is recorded: the GPU starts 0.35 ms earlier
+  // than behind the capture and instantiation of some 110 launches (16 jobs:
+  // 11.34 -> 10.99 ms a call)
+  if (tu.use_graph && waves > 1) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
-      record_batch_wave(lead, s, cfg, bt, bp.max_iter, bp.features, bp.max_items);
+      launches = record_batch_wave(lead, s, cfg, bt, bp.max_iter, bp.features, bp.lobes, bp.max_items);
     } catch (...) {
       cudaStreamEndCapture(s, &g);
       if (g)
@@ -1101,8 +1136,6 @@ void render_batch_impl(const phc_job *jobs, uint32_t n, phc_render_stats *out_st
       throw;
     }
     ck(cudaStreamEndCapture(s, &g), "end capture");
-    size_t nodes = 0;
-    cudaGraphGetNodes(g, nullptr, &nodes);
     const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
     ck(e, "graph instantiate");
@@ -1113,12 +1146,12 @@ void render_batch_impl(const phc_job *jobs, uint32_t n, phc_render_stats *out_st
         ck(le, "graph launch");
       }
     }
-    launches = uint64_t(waves) * (nodes > 0 ? nodes - 1 : 0); // minus the counter memset node
+    launches *= waves;
     ck(cudaStreamSynchronize(s), "batch");
     cudaGraphExecDestroy(ge);
   } else {
     for (uint32_t wv = 0; wv < waves; ++wv)
-      record_batch_wave(lead, s, cfg, bt, bp.max_iter, bp.features, bp.max_items);
+      launches += record_batch_wave(lead, s, cfg, bt, bp.max_iter, bp.features, bp.lobes, bp.max_items);
   }
   for (size_t j = 0; j < rs.size(); ++j)
     launch_resolve(s, accum(rs[j]), frame_of(rs[j]), plans[j].npix, plans[j].lanes, float(plans[j].rc.spp),

@@ -668,6 +668,16 @@ void build_instancing(const phc_pt_scene &pt, bool has_scene_tris, const float l
     s.prim_light_pdf.resize(s.prim_vidx.size() / 4, 0.f);
 }
 
+uint32_t lean_class_of(uint32_t lobes)
+{
+  uint32_t best = 0;
+  for (uint32_t c = 1; c < SHADE_CLASSES; ++c)
+    if ((lobes & ~SHADE_CLASS_LOBES[c]) == 0u &&
+        __builtin_popcount(SHADE_CLASS_LOBES[c]) < __builtin_popcount(SHADE_CLASS_LOBES[best]))
+      best = c;
+  return best;
+}
+
 void build_host_scene(const phc_scene_desc &in, HostScene &s)
 {
   s = HostScene{};
@@ -1402,8 +1412,11 @@ std::string DeviceScene::upload(const HostScene &h, cudaStream_t s)
     class_mask |= 1u << (m.shade_class % SHADE_CLASSES);
   shade_class_count = uint32_t(__builtin_popcount(class_mask));
   may_pass = false;
-  for (const DevMaterial &m : h.materials)
+  lobes = 0;
+  for (const DevMaterial &m : h.materials) {
     may_pass = may_pass || material_may_pass(m);
+    lobes |= material_lobes(m);
+  }
   table_floats[PHC_TABLE_MAJORANTS] = h.vol_majorants.size();
   table_floats[PHC_TABLE_ENV_MARGINAL] = h.env_marginal.size();
   table_floats[PHC_TABLE_ENV_CONDITIONAL] = h.env_conditional.size();

@@ -122,6 +122,10 @@ struct HostScene {
 
 void build_host_scene(const phc_scene_desc &in, HostScene &out);
 
+// The shading class with the fewest lobes that has all of `lobes` (0: every
+// lobe): the lean hit kernel for queues that are not sorted by class.
+uint32_t lean_class_of(uint32_t lobes);
+
 // Owns the device copies of a HostScene.
 struct DeviceScene {
   std::vector<void *> allocations;
@@ -130,6 +134,7 @@ struct DeviceScene {
   uint64_t node_bytes{0}, tri_bytes{0};
   uint64_t texel_count{0};
   uint32_t shade_class_count{0}; // distinct shading classes among the materials
+  uint32_t lobes{0};             // every lobe some material can have (material_lobes)
   bool may_pass{true};           // a path may go through a surface without a bounce (scene_may_pass)
   uint32_t bvh_depth{0};
   uint64_t table_floats[5]{}; // lengths of the tables phc_scene_table reads (PHC_TABLE_*)

@@ -350,8 +350,8 @@ __device__ __forceinline__ void shade_path(const RenderConst &rc, const DevScene
 #endif
 // CLS: the shading class (lean hit kernels only; 0 = every lobe).  With a
 // class-sorted hit queue (hq.cls_end) a class kernel shades its class's run
-// of it, with its own work counter; otherwise only class 0 runs, over the
-// whole queue.
+// of it, with its own work counter; otherwise one kernel shades the whole
+// queue: class 0, or hq.whole_class.
 template <bool FULL, int PART, bool BATCH, uint32_t CLS = 0>
 __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SHADE_MIN_BLOCKS_LEAN) k_shade(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
     PathSoA in, PathSoA out, const float4 *__restrict__ hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it,
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
   if (PART == 1 && hq.cls_end && sorted) {
     lo = CLS == 0 ? 0u : hq.cls_end[CLS * MAT_CLASS_BINS - 1];
     n = hq.cls_end[(CLS + 1) * MAT_CLASS_BINS - 1] - lo;
-  } else if (CLS != 0) {
+  } else if (CLS != 0 && hq.whole_class != CLS) {
     return;
   }
   uint32_t *fetch = CLS != 0 ? wc.at(WaveCounters::F_CLASS + CLS, it)

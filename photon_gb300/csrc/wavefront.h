@@ -174,6 +174,9 @@ struct HitQueues {
   // MAT_CLASS_BINS - 1]), shaded by that class's kernel.
   uint32_t classes = 0;
   const uint32_t *cls_end = nullptr;
+  // Not sorted by class: the class (not 0) whose kernel shades the whole hit
+  // queue, every material of the scene having its lobes at most.
+  uint32_t whole_class = 0;
 };
 constexpr uint32_t MAT_SORT_BINS = 1024; // materials map to bin = id % MAT_SORT_BINS
 constexpr uint32_t MAT_CLASS_BINS = MAT_SORT_BINS / SHADE_CLASSES; // sorting by class: bin = class * this + id % this
