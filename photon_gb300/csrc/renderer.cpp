@@ -1282,7 +1282,7 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
   const WaveCounters wc = wave_counters(r, max_iter);
   const LaunchCfg cfg = launch_cfg(r, slots);
   LaunchCfg acfg = cfg;
-  acfg.blocks_shade = r->sm_count * adj_shade_max_active_blocks(128);
+  acfg.blocks_shade = r->sm_count * adj_shade_max_active_blocks(ADJ_THREADS);
   const RenderConst *drc = r->adj_rc.as<RenderConst>();
   AdjointArgs a{};
   a.primal = r->acc.as<float4>();

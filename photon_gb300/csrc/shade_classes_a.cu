@@ -13,7 +13,7 @@ template <uint32_t C>
 void launch_cls(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it, HitQueues hq)
 {
-  k_shade<false, 1, false, C><<<c.blocks_shade_lean, 128, 0, s>>>(rc, sc, BatchTable{}, in, out, hits, sh, acc, wc, it,
+  k_shade<false, 1, false, C><<<(c.blocks_shade_lean * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, BatchTable{}, in, out, hits, sh, acc, wc, it,
       hq);
 }
 } // namespace

@@ -11,7 +11,7 @@ template <uint32_t C>
 void launch_cls_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, WaveCounters wc, int it, HitQueues hq)
 {
-  k_shade<false, 1, true, C><<<c.blocks_shade_lean, 128, 0, s>>>(nullptr, DevScene{}, bt, in, out, hits, sh, Accum{},
+  k_shade<false, 1, true, C><<<(c.blocks_shade_lean * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, DevScene{}, bt, in, out, hits, sh, Accum{},
       wc, it, hq);
 }
 } // namespace

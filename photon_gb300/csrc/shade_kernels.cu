@@ -133,20 +133,20 @@ void launch_shade(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, Dev
   const BatchTable none{};
   if (v.full) {
     if (v.part == 0)
-      k_shade<true, 0, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 0, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<true, 1, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 1, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 2)
-      k_shade<true, 2, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 2, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<true, 3, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 3, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
   } else {
     if (v.part == 0)
-      k_shade<false, 0, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 0, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<false, 1, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 1, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<false, 2, false><<<b, 128, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 2, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
   }
 }
 
@@ -158,18 +158,18 @@ void launch_shade_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, PathS
   const Accum acc{};
   if (v.full) {
     if (v.part == 0)
-      k_shade<true, 0, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 0, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<true, 1, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 1, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<true, 2, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 2, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
   } else {
     if (v.part == 0)
-      k_shade<false, 0, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 0, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<false, 1, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 1, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<false, 2, true><<<b, 128, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 2, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
   }
 }
 

@@ -338,12 +338,16 @@ __device__ __forceinline__ void shade_path(const RenderConst &rc, const DevScene
 
 // BATCH: the path's job (PathSoA::info.w bits 17..) selects scene, constants
 // and accumulators, and travels with the continued path and its shadow ray.
-// Minimum resident 128-thread blocks per SM that the register allocation
-// must allow, per variant.  Shading is latency-bound (scattered path-state,
-// material and texture loads); a capped register count with some spilling
-// keeps more warps resident and hides more of that latency.
+// Resident threads per SM that the register allocation must allow, per
+// variant, in units of 128.  Shading waits for scattered loads (path state,
+// materials, textures) and, unless a block's warps keep together (block_fetch),
+// for instructions.  Lean kernels: 16 / 12 / 8 units (32 / 40 / 64 registers)
+// measured 41.5 / 39.9 / 39.0 ms of shading on the 500K workload and 4.20 / 3.75 /
+// 3.30 ms in the box room (before the blocks worked in step, more warps hid more
+// of the instruction waits and 12 was the best); full kernels: 16 / 12 / 8 units
+// 5.9 / 6.1 / 6.9 ms on an adaptive frame through a volume.
 #ifndef PHC_SHADE_MIN_BLOCKS_LEAN
-#define PHC_SHADE_MIN_BLOCKS_LEAN 12
+#define PHC_SHADE_MIN_BLOCKS_LEAN 8
 #endif
 #ifndef PHC_SHADE_MIN_BLOCKS_FULL
 #define PHC_SHADE_MIN_BLOCKS_FULL 16
@@ -353,12 +357,12 @@ __device__ __forceinline__ void shade_path(const RenderConst &rc, const DevScene
 // of it, with its own work counter; otherwise one kernel shades the whole
 // queue: class 0, or hq.whole_class.
 template <bool FULL, int PART, bool BATCH, uint32_t CLS = 0>
-__global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SHADE_MIN_BLOCKS_LEAN) k_shade(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
+__global__ void __launch_bounds__(SHADE_THREADS, (FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SHADE_MIN_BLOCKS_LEAN) * 128 / SHADE_THREADS) k_shade(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
     PathSoA in, PathSoA out, const float4 *__restrict__ hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it,
     HitQueues hq)
 {
   static_assert(CLS == 0 || (PART == 1 && !FULL), "class kernels are lean hit kernels");
-  if (wave_failed(wc))
+  if (__syncthreads_or(wave_failed(wc))) // (the same answer in the whole block)
     return;
   const uint32_t n_all =
       PART == 0 ? *wc.at(WaveCounters::COUNT, it) : (PART == 1 ? *wc.at(WaveCounters::HCOUNT, it) : (PART == 2 ? *wc.at(WaveCounters::MCOUNT, it) : *wc.at(WaveCounters::VCOUNT, it)));
@@ -372,11 +376,12 @@ __global__ void __launch_bounds__(128, FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SH
   }
   uint32_t *fetch = CLS != 0 ? wc.at(WaveCounters::F_CLASS + CLS, it)
                              : wc.at(PART == 3 ? WaveCounters::F_VSHADE : (PART == 2 ? WaveCounters::F_MISS : WaveCounters::F_SHADE), it);
+  const uint32_t share = block_share(n);
   for (;;) {
-    const uint32_t base = warp_fetch(fetch);
+    const uint32_t base = block_fetch(fetch, share);
     if (base >= n)
       break;
-    const uint32_t j = base + lane_id();
+    const uint32_t j = threadIdx.x < share ? base + threadIdx.x : n;
     bool cont = false, has_sh = false;
     NextPath np;
     ShadowRec sr;

@@ -83,4 +83,27 @@ struct WarpFeed {
   }
 };
 
+// Blocks that work in step.  Shading code is far larger than the instruction
+// caches, and warps that run through it each at its own place wait for
+// instructions more than for anything else; the warps of one block, started
+// together on a batch of blockDim.x consecutive items, fetch it once for all.
+// Every thread of the block calls these.
+
+// Items a block takes at a time: all its threads', or whole warps' fewer when
+// the queue is too short to give every block of the grid that many.
+__device__ __forceinline__ uint32_t block_share(uint32_t n)
+{
+  const uint32_t even = ((n + gridDim.x - 1u) / gridDim.x + 31u) & ~31u;
+  return min(max(even, 32u), blockDim.x);
+}
+__device__ __forceinline__ uint32_t block_fetch(uint32_t *ctr, uint32_t k)
+{
+  __shared__ uint32_t base;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    base = atomicAdd(ctr, k);
+  __syncthreads();
+  return base;
+}
+
 } // namespace phc

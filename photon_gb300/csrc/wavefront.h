@@ -196,6 +196,12 @@ struct Frame {
   float4 *albedo;
 };
 
+// Threads per block of the shading kernels and of the adjoint's, whose blocks
+// work in step (block_fetch, warp_feed.cuh).  500K workload, shading per frame:
+// warps on their own 47.9 ms, blocks of 128 / 256 / 512 threads in step 41.5 /
+// 40.9 / 39.9 ms; the adjoint of the differentiable workload 9.6 ms, and 9.2 /
+// 8.9 / 9.0 ms with 256 / 384 / 640.
+constexpr int SHADE_THREADS = 512, ADJ_THREADS = 384;
 struct LaunchCfg {
   int blocks_trace, blocks_shade, blocks_raygen;
   int blocks_shade_lean; // grid of the lean shading variant (its own occupancy)
