@@ -629,6 +629,7 @@ void check_wave_error(uint32_t w, const WaveCounters &wc, cudaStream_t s)
 // adapt_lanes: paths of an adaptive wave and the bytes of its accumulator planes
 constexpr uint64_t ADAPT_PATHS = 1ull << 25;
 constexpr uint64_t ADAPT_PLANE_BYTES = 24ull << 30;
+constexpr size_t ADAPT_PATH_BYTES = 352; // queues, hits and accumulators of one path
 
 // What one render call of one renderer needs: its constants, sample lanes
 // and wave count; prepared (buffers sized, accumulators zeroed) on stream s.
@@ -700,14 +701,24 @@ RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg,
 // 2^24 411 / 488 / 477, 2^25 454 / 543 / 476.  A pixel whose gate closes in
 // mid-wave has up to 15 samples traced for nothing; over these frames that is
 // at most 1e-6 of the rays, since most closing pixels do so at the first gate.
-// Frames with no room for two samples keep one per wave.
-uint32_t adapt_lanes(const RenderConst &rc, uint64_t wave_paths)
+// Frames with no room for two samples keep one per wave.  Buffers that have to
+// grow for it stay within a quarter of the device's free memory, so that a
+// program with many renderers still has room for all of them.
+uint32_t adapt_lanes(const phc_renderer *r, const RenderConst &rc, uint64_t wave_paths)
 {
   const uint64_t paths = std::min(ADAPT_PATHS, wave_paths);
   uint32_t n = 1;
   while (n < ADAPT_MIN_SAMPLES && n < rc.spp && uint64_t(2 * n) * rc.npix <= paths &&
       uint64_t(2 * n) * rc.npix * 2 * rc.max_iter * 16 <= ADAPT_PLANE_BYTES)
     n *= 2;
+  auto planes = [&](uint32_t lanes) { return size_t(lanes) * rc.npix * 2 * rc.max_iter * 16; };
+  if (n > 1 && (planes(n) > r->ad_planes.bytes || size_t(n) * rc.npix > r->cap_paths)) {
+    size_t free_bytes = 0, total = 0;
+    ck(cudaMemGetInfo(&free_bytes, &total), "memory info");
+    const size_t room = free_bytes / 4 + r->ad_planes.bytes + r->cap_paths * ADAPT_PATH_BYTES;
+    while (n > 1 && planes(n) + size_t(n) * rc.npix * ADAPT_PATH_BYTES > room)
+      n /= 2;
+  }
   return n;
 }
 
@@ -757,7 +768,7 @@ JobPlan prepare_job(phc_renderer *r, const phc_camera &cam, const phc_settings &
     lanes = uint32_t(std::min<uint64_t>(rc.spp, std::max<uint64_t>(1, (target + npix - 1) / npix)));
     lanes = std::min<uint32_t>(lanes, std::max<uint32_t>(1u, uint32_t((1ull << 28) / npix)));
   } else {
-    lanes = adapt_lanes(rc, uint64_t(tu.wave_paths));
+    lanes = adapt_lanes(r, rc, uint64_t(tu.wave_paths));
     if (lanes > 1 && !ensure_adaptive(r, npix, lanes, int(rc.max_iter)))
       lanes = 1; // no room for the planes: one sample per wave
   }
