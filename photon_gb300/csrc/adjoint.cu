@@ -1146,7 +1146,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, PHC_ADJ_MIN_BLOCKS * 128 / ADJ_TH
     AdjPathSoA out, const float4 *__restrict__ hits, AdjShadowSoA sh, WaveCounters wc, int it, AdjointArgs a,
     HitQueues hq)
 {
-  if (__syncthreads_or(wave_failed(wc))) // a traversal warp stopped at its trip cap: its results are incomplete
+  if (block_failed(wc)) // a traversal warp stopped at its trip cap: its results are incomplete
     return;
   __shared__ float smat[MAX_SMEM_MATERIALS * NP];
   __shared__ float svol[MAX_VOLUMES * 4];
@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, PHC_ADJ_MIN_BLOCKS * 128 / ADJ_TH
 __global__ void __launch_bounds__(128) k_adj_resolve(const RenderConst *__restrict__ rcp, DevScene sc,
     AdjShadowSoA sh, AdjPathSoA next, WaveCounters wc, int it, AdjointArgs a)
 {
-  if (wave_failed(wc)) // a traversal warp stopped at its trip cap: its results are incomplete
+  if (block_failed(wc)) // a traversal warp stopped at its trip cap: its results are incomplete
     return;
   __shared__ float smat[MAX_SMEM_MATERIALS * NP];
   __shared__ float svol[MAX_VOLUMES * 4];

@@ -16,7 +16,7 @@ namespace {
 __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restrict__ rcp, DevScene sc, PathSoA in,
     const float4 *__restrict__ hits, WaveCounters wc, int it, HitQueues hq, unsigned long long *lookups)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   // persistent warps with refill: a lane whose ray is done takes a new one
   // once wc.vol_refill lanes of its warp are idle; every trip is at most
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
 __global__ void __launch_bounds__(256) k_vol_route(const float4 *__restrict__ hits, WaveCounters wc, int it,
     HitQueues hq)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   const uint32_t warps = gridDim.x * (blockDim.x / 32u);

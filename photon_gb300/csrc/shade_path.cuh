@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, (FULL ? PHC_SHADE_MIN_BLOCKS_FU
     HitQueues hq)
 {
   static_assert(CLS == 0 || (PART == 1 && !FULL), "class kernels are lean hit kernels");
-  if (__syncthreads_or(wave_failed(wc))) // (the same answer in the whole block)
+  if (block_failed(wc))
     return;
   const uint32_t n_all =
       PART == 0 ? *wc.at(WaveCounters::COUNT, it) : (PART == 1 ? *wc.at(WaveCounters::HCOUNT, it) : (PART == 2 ? *wc.at(WaveCounters::MCOUNT, it) : *wc.at(WaveCounters::VCOUNT, it)));

@@ -9,6 +9,16 @@ namespace phc {
 
 constexpr uint32_t EMISSION_ONLY = 0x80000000u;
 
+// wave_failed asked once for a whole block or a whole warp, by all of its
+// threads.  A kernel that runs beside another one of the wave can start while
+// that one sets the error word; threads that meet at a barrier, a vote or a
+// shared array later must not have read different answers.
+__device__ __forceinline__ bool block_failed(const WaveCounters &wc) { return __syncthreads_or(wave_failed(wc)) != 0; }
+__device__ __forceinline__ bool warp_failed(const WaveCounters &wc)
+{
+  return __any_sync(WARP_FULL, wave_failed(wc)) != 0;
+}
+
 // Reserves one output slot per lane with pred set, keeping lane order; all
 // lanes of the warp call it (ballot + popc prefix, one atomic per warp).
 __device__ __forceinline__ uint32_t warp_append(uint32_t *ctr, bool pred)

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) k_raygen(const RenderConst *__restrict__ 
 __global__ void __launch_bounds__(256) k_adapt_merge(const RenderConst *__restrict__ rcp, AdaptState ad, Accum lanes,
     WaveCounters wc, uint32_t npix, uint32_t slots, int max_iter, unsigned long long *accepted)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   const RenderConst &rc = *rcp;
   const uint32_t s0 = *wc.wave * rc.lanes;
@@ -305,7 +305,7 @@ template <bool COUNT, bool SPLIT, bool BATCH, bool INST = false>
 __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TRACE_MIN_BLOCKS) k_trace(DevScene sc, BatchTable bt, PathSoA in, float4 *__restrict__ hits,
     WaveCounters wc, int it, uint64_t *stats, uint32_t refill, HitQueues hq)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_TRACE, it);
@@ -456,7 +456,7 @@ template <bool BATCH>
 __global__ void __launch_bounds__(256) k_mat_hist(DevScene sc, BatchTable bt, const uint4 *__restrict__ info,
     const float4 *__restrict__ hits, HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
-  if (wave_failed(wc))
+  if (block_failed(wc))
     return;
   __shared__ uint32_t h[MAT_SORT_BINS];
   const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(256) k_mat_hist(DevScene sc, BatchTable bt, co
 // One block of MAT_SORT_BINS threads: bins[0..) counts -> bins[MAT_SORT_BINS..) starts.
 __global__ void __launch_bounds__(MAT_SORT_BINS) k_mat_scan(HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
-  if (wave_failed(wc))
+  if (block_failed(wc))
     return;
   __shared__ uint32_t t[MAT_SORT_BINS];
   if (*wc.at(WaveCounters::HCOUNT, it) < hq.sort_threshold)
@@ -501,7 +501,7 @@ template <bool BATCH>
 __global__ void __launch_bounds__(256) k_mat_scatter(DevScene sc, BatchTable bt, const uint4 *__restrict__ info,
     const float4 *__restrict__ hits, HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
-  if (wave_failed(wc))
+  if (block_failed(wc))
     return;
   __shared__ uint32_t cnt[MAT_SORT_BINS];
   const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
@@ -549,7 +549,7 @@ template <bool COUNT, bool BATCH, bool DEFER = false, bool INST = false>
 __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
     ShadowSoA sh, Accum acc_param, WaveCounters wc, int it, uint64_t *stats, uint32_t refill)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_SHADOW, it);
@@ -653,7 +653,7 @@ template <bool BATCH>
 __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__restrict__ rcp, DevScene sc,
     BatchTable bt, ShadowSoA sh, Accum acc_param, WaveCounters wc, int it, unsigned long long *lookups)
 {
-  if (wave_failed(wc))
+  if (warp_failed(wc))
     return;
   // the unoccluded shadow rays (tmax >= 0) of the iteration: ratio-tracking
   // transmittance (stream dimension 0x10000 + iteration) times the NEE
