@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
-  const uint32_t refill_at = min(wc.vol_refill, (per_warp + 1u) >> 1);
+  const uint32_t refill_at = refill_lanes(wc.vol_refill, per_warp);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   VolTrack s;

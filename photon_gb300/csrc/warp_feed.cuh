@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "warp_rules.h"
+
 namespace phc {
 
 constexpr uint32_t WARP_FULL = 0xffffffffu;
@@ -23,26 +25,10 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *ctr, uint32_t k = 32u)
   return __shfl_sync(WARP_FULL, base, 0);
 }
 
-// Rays that a warp of a persistent traversal or tracking kernel works on at a
-// time, for a queue of n rays and a grid of `warps`: 32, or the power of two
-// that still gives half of the grid's warps work when n is too short for
-// full ones.  Such a queue is bound by latency: a step of a full warp takes
-// as long as its slowest lane (on the 500K-triangle scene a lone ray's step
-// takes 0.42 us and each triangle test 0.34 us, and a full warp makes 2.7-3.7
-// tests in a row per step where a lane makes 0.4), and the idle schedulers
-// cost nothing.  Measured on a 640 x 360, 1-spp frame of that scene: closest
-// hits 0.89 -> 0.71 ms, shadow rays 0.52 -> 0.41 ms; an adaptive 811 x 613
-// frame through a volume (one sample of every pixel per wave) 139 -> 122 ms.
-// All of the grid's warps, or a quarter of them, instead of half measured 1%
-// and 2% slower there.  Shading kernels gain nothing from it (their warps
-// wait for instructions, which more warps fetch more often).
+// lanes_for this grid.
 __device__ __forceinline__ uint32_t spread_lanes(uint32_t n)
 {
-  const uint32_t warps = max(gridDim.x * (blockDim.x / 32u) / 2u, 1u);
-  uint32_t k = 1u;
-  while (k < 32u && k * warps < n)
-    k <<= 1;
-  return k;
+  return lanes_for(n, gridDim.x * (blockDim.x / 32u));
 }
 
 constexpr uint32_t FEED_CHUNK = 64;

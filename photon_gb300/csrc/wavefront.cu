@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
-  const uint32_t refill_at = min(refill, (per_warp + 1u) >> 1);
+  const uint32_t refill_at = refill_lanes(refill, per_warp);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   TravCounters ctr{0u, 0u};
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ 
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
-  const uint32_t refill_at = min(refill, (per_warp + 1u) >> 1);
+  const uint32_t refill_at = refill_lanes(refill, per_warp);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   TravCounters ctr{0u, 0u};
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__rest
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
   const uint32_t lanes_on = per_warp >= 32u ? WARP_FULL : (1u << per_warp) - 1u;
-  const uint32_t refill_at = min(wc.vol_refill, (per_warp + 1u) >> 1);
+  const uint32_t refill_at = refill_lanes(wc.vol_refill, per_warp);
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
   VolTrack s;
