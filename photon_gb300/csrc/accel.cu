@@ -42,10 +42,10 @@ int fail(int code, const std::string &m)
   return code;
 }
 
-// One ray per thread.  SHORT: a call of at most one batch of rays per warp gives
-// every warp its place in the grid, with fewer than 32 rays each when there
-// are not enough for half of the warps (spread_lanes), and reads no counter;
-// longer calls have persistent warps that take 32-ray batches from `fetch`.
+// One ray per thread.  SHORT: the warps of a call whose rays are all in flight
+// at once take them by their place in the grid, brief_lanes each, and read no
+// counter; longer calls have persistent warps that take 32-ray batches from
+// `fetch`.
 // 1,000 rays against a 6,000-triangle mesh 54 -> 43 us a call, 30,000 bounce
 // rays 93 -> 80 us; long calls keep their own kernel because the shared one cost
 // them 2% (its batch size and last batch in registers).  Refilling idle lanes
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(128) k_level_a(DevScene sc, const float *__res
       dst[k] = rec[k];
   };
   if (SHORT) {
-    const uint32_t per_warp = spread_lanes(n);
+    const uint32_t per_warp = brief_lanes(n, gridDim.x * (blockDim.x / 32u));
     const uint32_t i = (blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5)) * per_warp + lane_id();
     if (lane_id() < per_warp && i < n)
       trace(i);
@@ -141,8 +141,11 @@ __global__ void __launch_bounds__(128) k_level_a(DevScene sc, const float *__res
 
 constexpr int LEVEL_A_BLOCKS = 16; // per SM, of 128 threads
 
-// Whether n rays are at most one batch per warp (and need no batch counter).
-bool level_a_short(const phc_accel *a, uint32_t n) { return n <= uint32_t(a->sm_count * LEVEL_A_BLOCKS) * 4u * 32u; }
+// Whether a call of n rays needs no batch counter.
+bool level_a_short(const phc_accel *a, uint32_t n)
+{
+  return brief_lanes(n, uint32_t(a->sm_count * LEVEL_A_BLOCKS) * 4u) != 0u;
+}
 
 // The traversal of n > 0 rays on stream s; a long call's counter `fetch` is 0.
 template <int MODE, bool COUNT>

@@ -33,6 +33,26 @@ PHC_HD uint32_t lanes_for(uint32_t n, uint32_t warps)
   return k;
 }
 
+// Rays per warp of a ray back-end call that gives every warp its rays by its
+// place in the grid; 0 for longer calls, whose warps take batches from a
+// counter.  All rays of such a call must be in flight at once (half of the
+// grid's warps are resident): beyond, a block's place is only free again when
+// its last warp is done, and 160K-311K rays took 3-15% longer than from the
+// counter (200K random rays, 50K triangles: 206 and 226 us).  16 rays a
+// warp cost the issue slots of full warps and save little waiting: 45K-77K camera
+// rays on 6K triangles 80-91 us from the counter, 83-103 with 16, 72-81 with 32.
+// With 8, 30K rays on 500K triangles: camera rays 76 -> 61 us, any hit 53 -> 41
+// and 37 -> 35, incoherent closest hits 58 -> 60 (6K triangles: 79 -> 81, 74 -> 67,
+// 88 -> 89); with fewer, all calls gain (1,000 rays on 6K triangles 79 -> 51 us).
+PHC_HD uint32_t brief_lanes(uint32_t n, uint32_t warps)
+{
+  const uint32_t half = warps / 2u > 1u ? warps / 2u : 1u;
+  if (n > half * 32u)
+    return 0u;
+  const uint32_t k = lanes_for(n, warps);
+  return k <= 8u ? k : 32u;
+}
+
 // Idle lanes at which a warp that works on per_warp rays at a time takes new
 // ones: what the caller asked for (1..32; 32: only when all are idle), but no
 // more than half of the rays of a warp that has fewer than 32.

@@ -21,7 +21,7 @@ def lib(tmp_path_factory):
                     "-I", os.path.join(ROOT, "photon_gb300", "csrc"),
                     os.path.join(ROOT, "tests", "native", "warp_rules_test.cpp"), "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
-    for f in ("wr_lanes_for", "wr_refill_lanes"):
+    for f in ("wr_lanes_for", "wr_refill_lanes", "wr_brief_lanes"):
         getattr(lib, f).restype = C.c_uint32
         getattr(lib, f).argtypes = [C.c_uint32, C.c_uint32]
     return lib
@@ -46,3 +46,17 @@ def test_spread_queues_are_covered(lib, warps):
         assert k in (1, 2, 4, 8, 16, 32)
         assert k == 32 or k * half >= n      # half of the warps hold the whole queue
         assert k == 1 or (k // 2) * half < n  # with no more lanes than that takes
+
+
+@pytest.mark.parametrize("warps", [1, 2, 64, 2432, 9728])
+def test_short_calls_are_all_in_flight(lib, warps):
+    """Rays go by the warps' places only while half of the grid (what is
+    resident) holds them all, and never with 16 lanes of a warp on."""
+    half = max(warps // 2, 1)
+    for n in [1, half, half + 1, 2 * half, 4 * half, 8 * half, 8 * half + 1, 16 * half, 16 * half + 1, 32 * half]:
+        k = lib.wr_brief_lanes(n, warps)
+        assert k in (1, 2, 4, 8, 32)
+        assert k * half >= n
+        assert k == 32 or k == 1 or (k // 2) * half < n
+    for n in [32 * half + 1, 64 * half - 1, 64 * half, 2 ** 30]:
+        assert lib.wr_brief_lanes(n, warps) == 0
