@@ -1203,10 +1203,15 @@ __global__ void __launch_bounds__(ADJ_THREADS, PHC_ADJ_MIN_BLOCKS * 128 / ADJ_TH
   end_grads(g, sc, a);
 }
 
+// Its grid is what its own 72 registers leave resident (7 blocks per SM): the
+// adjoint through a volume, 512 x 512 at 16 spp, takes 42.8 ms, 46.4 with the 3
+// blocks per SM of k_adj_shade's larger ones, and 10, 14 or 21 change nothing.
+constexpr int ADJ_RESOLVE_THREADS = 128;
+
 // The shadow rays of one bounce after k_shadow (deferred mode): for each
 // unoccluded one the transmittance (with its derivative), the contribution
 // collected, the continued path's remainder reduced, the vertex's gradient.
-__global__ void __launch_bounds__(128) k_adj_resolve(const RenderConst *__restrict__ rcp, DevScene sc,
+__global__ void __launch_bounds__(ADJ_RESOLVE_THREADS) k_adj_resolve(const RenderConst *__restrict__ rcp, DevScene sc,
     AdjShadowSoA sh, AdjPathSoA next, WaveCounters wc, int it, AdjointArgs a)
 {
   if (block_failed(wc)) // a traversal warp stopped at its trip cap: its results are incomplete
@@ -1285,10 +1290,10 @@ void launch_adj_shade(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc,
   k_adj_shade<<<c.blocks_shade, ADJ_THREADS, 0, s>>>(rc, sc, in, out, hits, sh, wc, it, a, hq);
 }
 
-void launch_adj_resolve(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, AdjShadowSoA sh,
+void launch_adj_resolve(int blocks, cudaStream_t s, const RenderConst *rc, DevScene sc, AdjShadowSoA sh,
     AdjPathSoA next, WaveCounters wc, int it, AdjointArgs a)
 {
-  k_adj_resolve<<<c.blocks_shade, 128, 0, s>>>(rc, sc, sh, next, wc, it, a);
+  k_adj_resolve<<<blocks, ADJ_RESOLVE_THREADS, 0, s>>>(rc, sc, sh, next, wc, it, a);
 }
 
 void launch_adj_finish(cudaStream_t s, int blocks, uint32_t slots, AdjointArgs a)
@@ -1296,12 +1301,17 @@ void launch_adj_finish(cudaStream_t s, int blocks, uint32_t slots, AdjointArgs a
   k_adj_finish<<<blocks, 256, 0, s>>>(slots, a);
 }
 
-int adj_shade_max_active_blocks(int threads)
+namespace {
+template <class K> int resident_blocks(K kernel, int threads)
 {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_shade, threads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess)
     return 1;
   return n > 0 ? n : 1;
 }
+} // namespace
+
+int adj_shade_blocks_per_sm() { return resident_blocks(k_adj_shade, ADJ_THREADS); }
+int adj_resolve_blocks_per_sm() { return resident_blocks(k_adj_resolve, ADJ_RESOLVE_THREADS); }
 
 } // namespace phc

@@ -63,9 +63,13 @@ struct AdjointArgs {
 void launch_adj_shade(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, AdjPathSoA in,
     AdjPathSoA out, const float4 *hits, AdjShadowSoA sh, WaveCounters wc, int it, AdjointArgs a,
     HitQueues hq);
-void launch_adj_resolve(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, AdjShadowSoA sh,
+// blocks: a grid of its own (adj_resolve_blocks_per_sm), for the next bounce's
+// shading waits for it.
+void launch_adj_resolve(int blocks, cudaStream_t s, const RenderConst *rc, DevScene sc, AdjShadowSoA sh,
     AdjPathSoA next, WaveCounters wc, int it, AdjointArgs a);
 void launch_adj_finish(cudaStream_t s, int blocks, uint32_t slots, AdjointArgs a);
-int adj_shade_max_active_blocks(int threads);
+// Resident blocks per SM of the two kernels above at their block sizes.
+int adj_shade_blocks_per_sm();
+int adj_resolve_blocks_per_sm();
 
 } // namespace phc

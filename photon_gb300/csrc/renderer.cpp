@@ -1293,7 +1293,8 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
   const WaveCounters wc = wave_counters(r, max_iter);
   const LaunchCfg cfg = launch_cfg(r, slots);
   LaunchCfg acfg = cfg;
-  acfg.blocks_shade = r->sm_count * adj_shade_max_active_blocks(ADJ_THREADS);
+  acfg.blocks_shade = r->sm_count * adj_shade_blocks_per_sm();
+  const int resolve_blocks = r->sm_count * adj_resolve_blocks_per_sm();
   const RenderConst *drc = r->adj_rc.as<RenderConst>();
   AdjointArgs a{};
   a.primal = r->acc.as<float4>();
@@ -1348,7 +1349,7 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
       launch_adj_shade(acfg, s, drc, sc, in, out, hits, q.shadow, wc, it, a, rq);
       const cudaStream_t ss = shadows.begin();
       launch_shadow_deferred(cfg, ss, sc, q.shadow.s, wc, it, tu.trace_refill);
-      launch_adj_resolve(acfg, ss, drc, sc, q.shadow, out, wc, it, a);
+      launch_adj_resolve(resolve_blocks, ss, drc, sc, q.shadow, out, wc, it, a);
       shadows.end();
     }
     shadows.join();
