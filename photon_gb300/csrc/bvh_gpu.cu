@@ -1152,14 +1152,25 @@ struct DeviceLimits {
   int sms{0}, ploc_blocks{0}, collapse_blocks{0};
 };
 
-// Grid limits of the cooperative kernels on the current device.
-DeviceLimits device_limits()
+// The clustering kernel of a search radius.
+const void *ploc_kernel(int radius)
+{
+  return radius <= 2 ? (const void *)k_ploc<2>
+      : radius <= 4  ? (const void *)k_ploc<4>
+      : radius <= 8  ? (const void *)k_ploc<8>
+      : radius <= 16 ? (const void *)k_ploc<16>
+                     : (const void *)k_ploc<32>;
+}
+
+// Grid limits of the cooperative kernels on the current device: the clustering
+// kernel that will be launched, and the collapse.
+DeviceLimits device_limits(const void *ploc)
 {
   DeviceLimits d;
   int dev = 0;
   ck(cudaGetDevice(&dev), "device");
   ck(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev), "device");
-  ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.ploc_blocks, k_ploc<32>, PLOC_BLOCK, 0), "occupancy");
+  ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.ploc_blocks, ploc, PLOC_BLOCK, 0), "occupancy");
   ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.collapse_blocks, k_collapse_sah, COLLAPSE_BLOCK, 0),
       "occupancy");
   return d;
@@ -1174,13 +1185,16 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
     throw std::runtime_error("gpu bvh build: no triangles");
   if (n > (1u << 30))
     throw std::runtime_error("gpu bvh build: too many triangles");
-  const DeviceLimits lim = device_limits();
+  const void *ploc = ploc_kernel(radius);
+  const DeviceLimits lim = device_limits(ploc);
   const uint32_t nb = (n + SORT_BLOCK - 1) / SORT_BLOCK;
   const uint32_t nodes2 = 2 * n - 1, inner = n - 1;
   const bool program = tri_cost > 0.f && inner > 0;
   const int leaf_max = std::min(std::max(max_leaf, 1), 3);
   const uint32_t ploc_blocks =
-      n <= PLOC_ALONE ? 1u : std::min<uint32_t>(uint32_t(lim.sms * std::min(std::max(lim.ploc_blocks, 1), PLOC_BLOCKS_PER_SM)), (n + PLOC_BLOCK - 1) / PLOC_BLOCK);
+      n <= PLOC_ALONE ? 1u
+                      : std::min<uint32_t>(uint32_t(lim.sms * std::min(std::max(lim.ploc_blocks, 1), PLOC_BLOCKS_PER_SM)),
+                            (n + PLOC_BLOCK - 1) / PLOC_BLOCK);
   Scratch sc;
   float *boxes, *nbox;
   uint32_t *cb, *keys[2], *vals[2], *hist, *scan_tmp, *ctr, *nodes_big;
@@ -1243,12 +1257,7 @@ GpuBvh8 build_bvh8_gpu(const float4 *positions, const uint4 *prim_vidx, uint32_t
   ck(cudaMemsetAsync(job.result, 0, 16, s), "clustering result");
   {
     void *args[] = {&job};
-    const void *kernel = radius <= 2 ? (const void *)k_ploc<2>
-        : radius <= 4                ? (const void *)k_ploc<4>
-        : radius <= 8                ? (const void *)k_ploc<8>
-        : radius <= 16               ? (const void *)k_ploc<16>
-                                     : (const void *)k_ploc<32>;
-    ck(cudaLaunchCooperativeKernel(kernel, dim3(ploc_blocks), dim3(PLOC_BLOCK), args, 0, s), "clustering launch");
+    ck(cudaLaunchCooperativeKernel(ploc, dim3(ploc_blocks), dim3(PLOC_BLOCK), args, 0, s), "clustering launch");
   }
   uint32_t result[4];
   ck(cudaMemcpyAsync(result, job.result, 16, cudaMemcpyDeviceToHost, s), "read clustering");
