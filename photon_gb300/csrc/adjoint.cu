@@ -1142,7 +1142,8 @@ __device__ __forceinline__ void adj_shade_path(const RenderConst &rc, const DevS
 // sorted by material when there are at least hq.sort_threshold of them; the
 // paths are then replayed hits first, in that order, then the misses, so
 // that a warp's lanes mostly run one material's code.
-__global__ void __launch_bounds__(ADJ_THREADS, PHC_ADJ_MIN_BLOCKS * 128 / ADJ_THREADS) k_adj_shade(const RenderConst *__restrict__ rcp, DevScene sc, AdjPathSoA in,
+__global__ void __launch_bounds__(ADJ_THREADS, PHC_ADJ_MIN_BLOCKS * 128 / ADJ_THREADS)
+k_adj_shade(const RenderConst *__restrict__ rcp, DevScene sc, AdjPathSoA in,
     AdjPathSoA out, const float4 *__restrict__ hits, AdjShadowSoA sh, WaveCounters wc, int it, AdjointArgs a,
     HitQueues hq)
 {

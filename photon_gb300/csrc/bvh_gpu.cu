@@ -308,17 +308,18 @@ __global__ void k_leaves(const float *__restrict__ boxes, const uint32_t *__rest
   }
 }
 
-// The whole clustering in one cooperative launch.  It used to be ten launches
-// and a read of two counters per iteration, 45-58 iterations of mostly a few
-// hundred clusters: 2.4 of the 4.6 ms that a 50K-triangle build took.  Here an
+// The whole clustering in one cooperative launch: 45-58 iterations of mostly a
+// few hundred clusters each, which as launches of their own (ten, and a read of
+// two counters) take 2.4 ms for 50K triangles, in whole builds of 4.6 and 1.5 ms.  An
 // iteration is three phases between grid barriers (neighbours; merges and
 // survivors counted per block; ranks and output), and once the clusters fit
 // one block (PLOC_ALONE), it goes on alone with them in shared memory.  The
 // surface-area program of the nodes an iteration made runs with the next
 // one's neighbour search (their children are older, so their entries are
 // final).  Measured whole builds (968 / 63,368 triangles): blocks of 256, 512 and
-// 1024 threads within 5% of one another, 512 with two per SM the fastest.  Ranks are exact integer prefix sums in cluster order, so the tree and
-// its numbering do not depend on the grid.
+// 1024 threads within 5% of one another, 512 with two per SM the fastest.  Ranks
+// are exact integer prefix sums in cluster order, so the tree and its numbering
+// do not depend on the grid.
 constexpr int PLOC_BLOCK = 512;
 constexpr int PLOC_BLOCKS_PER_SM = 2;
 constexpr uint32_t PLOC_ALONE = PLOC_BLOCK;
@@ -795,12 +796,11 @@ __global__ void __launch_bounds__(128) k_collapse(Collapse c, const uint2 *__res
 
 // ---------------------------------------------------------------- stage 4a
 // The collapse by the surface-area program (bvh_collapse.cuh): every level of
-// the wide tree in one cooperative launch, eight lanes per wide node.  With one
-// thread per node and one launch and counter read per level, a level took
-// 60-100 us however few nodes it had (the octant slots are a greedy choice
-// among 64 costs, then 48 quantised planes); the eight lanes hold one child,
-// then one slot, each, and a level takes about 15 us.  With the clustering in
-// one launch (k_ploc) a 52K-triangle mesh is built in 1.5 ms instead of 4.6.
+// the wide tree in one cooperative launch, eight lanes per wide node, which
+// hold one child, then one slot, each (the octant slots are a greedy choice
+// among 64 costs, then come 48 quantised planes).  A level takes about 15 us;
+// with one thread per node and a launch and counter read per level it takes
+// 60-100 us however few nodes it has.
 struct CollapseSah {
   const uint8_t *split; // CollapseDp::split
   const uchar4 *info;   // CollapseDp::info

@@ -713,9 +713,12 @@ RenderConst render_const(const phc_camera &cam, const phc_settings &st, Buf &bg,
 // even 3.7M paths (1920 x 1920) do.  Measured through the 2M-triangle volume
 // scene at 64 spp (Msamples/s; 1920 x 1920, 1920 x 1080, 1280 x 720): one
 // sample per wave 260 / 205 / 115; waves of up to 2^23 paths 342 / 402 / 386,
-// 2^24 411 / 488 / 477, 2^25 454 / 543 / 476.  A pixel whose gate closes in
-// mid-wave has up to 15 samples traced for nothing; over these frames that is
-// at most 1e-6 of the rays, since most closing pixels do so at the first gate.
+// 2^24 411 / 488 / 477, 2^25 454 / 543 / 476.  Samples that the gate refuses in
+// mid-wave are traced for nothing, but they are few: most closing pixels are
+// black and close at the first gate, before a wave; any other's refused sample
+// adds a square to its sums of squares (adapt_square), some 1/n of them after n
+// samples, which opens the gate again while n is below about 100.  Over these
+// frames they are at most 1e-6 of the rays.
 // Frames with no room for two samples keep one per wave.  Buffers that have to
 // grow for it stay within a quarter of the device's free memory, so that a
 // program with many renderers still has room for all of them.

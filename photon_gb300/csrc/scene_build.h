@@ -135,7 +135,7 @@ struct DeviceScene {
   uint64_t texel_count{0};
   uint32_t shade_class_count{0}; // distinct shading classes among the materials
   uint32_t lobes{0};             // every lobe some material can have (material_lobes)
-  bool may_pass{true};           // a path may go through a surface without a bounce (scene_may_pass)
+  bool may_pass{true};           // a path may go through a surface without a bounce (material_may_pass)
   uint32_t bvh_depth{0};
   uint64_t table_floats[5]{}; // lengths of the tables phc_scene_table reads (PHC_TABLE_*)
   void *aux{nullptr};         // AUX_BYTES of device memory for the scene's owner

@@ -8,8 +8,8 @@ template <uint32_t C>
 void launch_cls(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it, HitQueues hq)
 {
-  k_shade<false, 1, false, C><<<(c.blocks_shade_lean * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, BatchTable{}, in, out, hits, sh, acc, wc, it,
-      hq);
+  k_shade<false, 1, false, C><<<shade_grid(c.blocks_shade_lean), SHADE_THREADS, 0, s>>>(rc, sc, BatchTable{}, in, out, hits,
+      sh, acc, wc, it, hq);
 }
 } // namespace
 

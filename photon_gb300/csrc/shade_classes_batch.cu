@@ -11,8 +11,8 @@ template <uint32_t C>
 void launch_cls_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, WaveCounters wc, int it, HitQueues hq)
 {
-  k_shade<false, 1, true, C><<<(c.blocks_shade_lean * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, DevScene{}, bt, in, out, hits, sh, Accum{},
-      wc, it, hq);
+  k_shade<false, 1, true, C><<<shade_grid(c.blocks_shade_lean), SHADE_THREADS, 0, s>>>(nullptr, DevScene{}, bt, in, out,
+      hits, sh, Accum{}, wc, it, hq);
 }
 } // namespace
 

@@ -129,47 +129,47 @@ void launch_vol_scatter(const LaunchCfg &c, cudaStream_t s, const RenderConst *r
 void launch_shade(const LaunchCfg &c, cudaStream_t s, const RenderConst *rc, DevScene sc, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it, ShadeVariant v, HitQueues hq)
 {
-  const int b = v.full ? c.blocks_shade : c.blocks_shade_lean;
+  const int b = shade_grid(v.full ? c.blocks_shade : c.blocks_shade_lean);
   const BatchTable none{};
   if (v.full) {
     if (v.part == 0)
-      k_shade<true, 0, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 0, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<true, 1, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 1, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 2)
-      k_shade<true, 2, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 2, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<true, 3, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 3, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
   } else {
     if (v.part == 0)
-      k_shade<false, 0, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 0, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<false, 1, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 1, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<false, 2, false><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 2, false><<<b, SHADE_THREADS, 0, s>>>(rc, sc, none, in, out, hits, sh, acc, wc, it, hq);
   }
 }
 
 void launch_shade_batch(const LaunchCfg &c, cudaStream_t s, BatchTable bt, PathSoA in, PathSoA out,
     const float4 *hits, ShadowSoA sh, WaveCounters wc, int it, ShadeVariant v, HitQueues hq)
 {
-  const int b = v.full ? c.blocks_shade : c.blocks_shade_lean;
+  const int b = shade_grid(v.full ? c.blocks_shade : c.blocks_shade_lean);
   const DevScene sc{};
   const Accum acc{};
   if (v.full) {
     if (v.part == 0)
-      k_shade<true, 0, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 0, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<true, 1, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 1, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<true, 2, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<true, 2, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
   } else {
     if (v.part == 0)
-      k_shade<false, 0, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 0, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else if (v.part == 1)
-      k_shade<false, 1, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 1, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
     else
-      k_shade<false, 2, true><<<(b * 128 + SHADE_THREADS - 1) / SHADE_THREADS, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
+      k_shade<false, 2, true><<<b, SHADE_THREADS, 0, s>>>(nullptr, sc, bt, in, out, hits, sh, acc, wc, it, hq);
   }
 }
 

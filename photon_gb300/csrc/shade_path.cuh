@@ -343,9 +343,8 @@ __device__ __forceinline__ void shade_path(const RenderConst &rc, const DevScene
 // materials, textures) and, unless a block's warps keep together (block_fetch),
 // for instructions.  Lean kernels: 16 / 12 / 8 units (32 / 40 / 64 registers)
 // measured 41.5 / 39.9 / 39.0 ms of shading on the 500K workload and 4.20 / 3.75 /
-// 3.30 ms in the box room (before the blocks worked in step, more warps hid more
-// of the instruction waits and 12 was the best); full kernels: 16 / 12 / 8 units
-// 5.9 / 6.1 / 6.9 ms on an adaptive frame through a volume.
+// 3.30 ms in the box room; full kernels: 16 / 12 / 8 units 5.9 / 6.1 / 6.9 ms on
+// an adaptive frame through a volume.
 #ifndef PHC_SHADE_MIN_BLOCKS_LEAN
 #define PHC_SHADE_MIN_BLOCKS_LEAN 8
 #endif
@@ -357,15 +356,18 @@ __device__ __forceinline__ void shade_path(const RenderConst &rc, const DevScene
 // of it, with its own work counter; otherwise one kernel shades the whole
 // queue: class 0, or hq.whole_class.
 template <bool FULL, int PART, bool BATCH, uint32_t CLS = 0>
-__global__ void __launch_bounds__(SHADE_THREADS, (FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SHADE_MIN_BLOCKS_LEAN) * 128 / SHADE_THREADS) k_shade(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
-    PathSoA in, PathSoA out, const float4 *__restrict__ hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it,
-    HitQueues hq)
+__global__ void __launch_bounds__(SHADE_THREADS,
+    (FULL ? PHC_SHADE_MIN_BLOCKS_FULL : PHC_SHADE_MIN_BLOCKS_LEAN) * 128 / SHADE_THREADS)
+k_shade(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt, PathSoA in, PathSoA out,
+    const float4 *__restrict__ hits, ShadowSoA sh, Accum acc, WaveCounters wc, int it, HitQueues hq)
 {
   static_assert(CLS == 0 || (PART == 1 && !FULL), "class kernels are lean hit kernels");
   if (block_failed(wc))
     return;
-  const uint32_t n_all =
-      PART == 0 ? *wc.at(WaveCounters::COUNT, it) : (PART == 1 ? *wc.at(WaveCounters::HCOUNT, it) : (PART == 2 ? *wc.at(WaveCounters::MCOUNT, it) : *wc.at(WaveCounters::VCOUNT, it)));
+  constexpr uint32_t QUEUE[4] = {WaveCounters::COUNT, WaveCounters::HCOUNT, WaveCounters::MCOUNT, WaveCounters::VCOUNT};
+  constexpr uint32_t FETCH[4] = {WaveCounters::F_SHADE, WaveCounters::F_SHADE, WaveCounters::F_MISS,
+      WaveCounters::F_VSHADE};
+  const uint32_t n_all = *wc.at(QUEUE[PART], it);
   const bool sorted = PART == 1 && hq.sort_threshold != 0u && n_all >= hq.sort_threshold;
   uint32_t lo = 0, n = n_all;
   if (PART == 1 && hq.cls_end && sorted) {
@@ -374,8 +376,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, (FULL ? PHC_SHADE_MIN_BLOCKS_FU
   } else if (CLS != 0 && hq.whole_class != CLS) {
     return;
   }
-  uint32_t *fetch = CLS != 0 ? wc.at(WaveCounters::F_CLASS + CLS, it)
-                             : wc.at(PART == 3 ? WaveCounters::F_VSHADE : (PART == 2 ? WaveCounters::F_MISS : WaveCounters::F_SHADE), it);
+  uint32_t *fetch = wc.at(CLS != 0 ? WaveCounters::F_CLASS + CLS : FETCH[PART], it);
   const uint32_t share = block_share(n);
   for (;;) {
     const uint32_t base = block_fetch(fetch, share);

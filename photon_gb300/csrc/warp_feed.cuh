@@ -44,8 +44,9 @@ constexpr uint32_t FEED_CHUNK = 64;
 struct WarpFeed {
   uint32_t cur{0}, end{0}, chunk;
   bool last{false}; // the counter has run past n
-  // per_warp: items the warp works on at a time (spread_lanes).  A chunk is at
-  // most an eighth of a warp's share, so that the launch's end stays even.
+  // per_warp: items the warp works on at a time (spread_lanes).  A full warp's
+  // chunk is an eighth of its share, so that the launch's end stays even, but
+  // at least 32 and at most FEED_CHUNK items.
   __device__ __forceinline__ WarpFeed(uint32_t n, uint32_t per_warp)
   {
     const uint32_t share = n / (gridDim.x * (blockDim.x / 32u) * 8u);

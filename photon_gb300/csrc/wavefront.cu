@@ -383,7 +383,8 @@ __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TR
       const uint32_t hm = __ballot_sync(WARP_FULL, is_hit);
       const uint32_t mm = dm & ~hm;
       if (done)
-        out[is_hit ? 0 : 1][((is_hit ? h_at + h_n : m_at + m_n) + uint32_t(__popc((is_hit ? hm : mm) & lt_mask))) & 63u] = idx;
+        out[is_hit ? 0 : 1]
+           [((is_hit ? h_at + h_n : m_at + m_n) + uint32_t(__popc((is_hit ? hm : mm) & lt_mask))) & 63u] = idx;
       h_n += uint32_t(__popc(hm));
       m_n += uint32_t(__popc(mm));
       __syncwarp();

@@ -202,6 +202,8 @@ struct Frame {
 // 40.9 / 39.9 ms; the adjoint of the differentiable workload 9.6 ms, and 9.2 /
 // 8.9 / 9.0 ms with 256 / 384 / 640.
 constexpr int SHADE_THREADS = 512, ADJ_THREADS = 384;
+// The grid of a shading kernel, from its size in 128-thread blocks.
+constexpr int shade_grid(int blocks) { return (blocks * 128 + SHADE_THREADS - 1) / SHADE_THREADS; }
 struct LaunchCfg {
   int blocks_trace, blocks_shade, blocks_raygen;
   int blocks_shade_lean; // grid of the lean shading variant (its own occupancy)
