@@ -378,21 +378,6 @@ struct KernelTimer {
   }
 };
 
-// The side streams and their events, made for the first waves that a renderer
-// launches (a batch's other renderers launch none, and a renderer is made in
-// 3 us without them, in 7.5 with them).
-void ensure_sides(phc_renderer *r)
-{
-  for (int k = 0; k < phc_renderer::SIDES; ++k) {
-    if (!r->side[k])
-      ck(cudaStreamCreateWithFlags(&r->side[k], cudaStreamNonBlocking), "cudaStreamCreate");
-    if (!r->fork_ev[k])
-      ck(cudaEventCreateWithFlags(&r->fork_ev[k], cudaEventDisableTiming), "cudaEventCreate");
-    if (!r->join_ev[k])
-      ck(cudaEventCreateWithFlags(&r->join_ev[k], cudaEventDisableTiming), "cudaEventCreate");
-  }
-}
-
 // Whether a wave of this many paths sorts its hit queues at all.
 bool sorts_wave(const Tuning &tu, uint64_t wave_paths)
 {
@@ -526,7 +511,7 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
   if (tm)
     tm->begin_wave();
   timed(0, [&] { launch_raygen(cfg, s, rc, sc, path_soa(r, 0), acc_all, wc, ad); });
-  SideBranch shadows(r, s, 0, tm == nullptr), part_a(r, s, 1, tm == nullptr), part_b(r, s, 2, tm == nullptr);
+    SideBranch shadows(r, s, 0, tm == nullptr), part_a(r, s, 1, tm == nullptr), part_b(r, s, 2, tm == nullptr);
   for (int it = 0; it < max_iter; ++it) {
     const PathSoA in = path_soa(r, it & 1), out = path_soa(r, (it + 1) & 1);
     float4 *hits = r->hits.as<float4>();
@@ -856,7 +841,6 @@ void render_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st,
   const int max_iter = plan.max_iter;
   const bool first = plan.first;
   const Tuning &tu = tuning();
-  ensure_sides(r);
   ensure_paths(r, plan.slots);
   ensure_wave_buffers(r, max_iter);
   ck(cudaMemsetAsync(r->stats_buf.p, 0, 8 * sizeof(uint64_t), s), "reset stats");
@@ -1136,7 +1120,6 @@ void render_batch_impl(const phc_job *jobs, uint32_t n, phc_render_stats *out_st
   upload_vec(lead->b_entries, bp.entries, s, "upload batch entries");
   upload_vec(lead->b_wave_entry, bp.wave_entry, s, "upload batch waves");
   upload_vec(lead->b_wave_items, bp.wave_items, s, "upload batch waves");
-  ensure_sides(lead);
   ensure_paths(lead, bp.max_items);
   ensure_wave_buffers(lead, bp.max_iter);
   ck(lead->sh_job.ensure(size_t(std::max<uint32_t>(bp.max_items, 1)) * 4), "alloc shadow jobs");
@@ -1287,7 +1270,6 @@ void adjoint_impl(phc_renderer *r, const phc_camera &cam, const phc_settings &st
   const uint64_t per_chunk = std::max<uint64_t>(uint64_t(tu.wave_paths), npix);
   const uint32_t chunk = uint32_t(std::min<uint64_t>(spp, std::max<uint64_t>(1, per_chunk / npix)));
   const size_t slots = size_t(chunk) * npix;
-  ensure_sides(r);
   ensure_slots(r, slots);
   ensure_paths(r, slots);
   ensure_wave_buffers(r, max_iter);
@@ -1534,6 +1516,11 @@ int phc_create(phc_renderer **out)
     ck(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     ck(cudaEventCreate(&r->ev0), "cudaEventCreate");
     ck(cudaEventCreate(&r->ev1), "cudaEventCreate");
+    for (int k = 0; k < phc_renderer::SIDES; ++k) {
+      ck(cudaStreamCreateWithFlags(&r->side[k], cudaStreamNonBlocking), "cudaStreamCreate");
+      ck(cudaEventCreateWithFlags(&r->fork_ev[k], cudaEventDisableTiming), "cudaEventCreate");
+      ck(cudaEventCreateWithFlags(&r->join_ev[k], cudaEventDisableTiming), "cudaEventCreate");
+    }
   });
   if (rc != PHC_OK) {
     delete r;
