@@ -511,7 +511,7 @@ uint64_t record_wave(phc_renderer *r, cudaStream_t s, const LaunchCfg &cfg, cons
   if (tm)
     tm->begin_wave();
   timed(0, [&] { launch_raygen(cfg, s, rc, sc, path_soa(r, 0), acc_all, wc, ad); });
-    SideBranch shadows(r, s, 0, tm == nullptr), part_a(r, s, 1, tm == nullptr), part_b(r, s, 2, tm == nullptr);
+  SideBranch shadows(r, s, 0, tm == nullptr), part_a(r, s, 1, tm == nullptr), part_b(r, s, 2, tm == nullptr);
   for (int it = 0; it < max_iter; ++it) {
     const PathSoA in = path_soa(r, it & 1), out = path_soa(r, (it + 1) & 1);
     float4 *hits = r->hits.as<float4>();

@@ -16,13 +16,13 @@ namespace {
 __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restrict__ rcp, DevScene sc, PathSoA in,
     const float4 *__restrict__ hits, WaveCounters wc, int it, HitQueues hq, unsigned long long *lookups)
 {
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   if (warp_failed(wc))
     return;
   // persistent warps with refill: a lane whose ray is done takes a new one
   // once wc.vol_refill lanes of its warp are idle; every trip is at most
   // wc.vol_passes passes of every busy lane's tracking (vt_pass: a macro-cell
   // step or a density lookup), ending at its next lookup
-  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_VSCATTER, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
@@ -91,9 +91,9 @@ __global__ void __launch_bounds__(128) k_vol_scatter(const RenderConst *__restri
 __global__ void __launch_bounds__(256) k_vol_route(const float4 *__restrict__ hits, WaveCounters wc, int it,
     HitQueues hq)
 {
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   if (warp_failed(wc))
     return;
-  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   const uint32_t warps = gridDim.x * (blockDim.x / 32u);
   for (uint32_t base = (blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5)) * 32u; base < n; base += warps * 32u) {
     const uint32_t i = base + lane_id();

@@ -12,7 +12,9 @@ constexpr uint32_t EMISSION_ONLY = 0x80000000u;
 // wave_failed asked once for a whole block or a whole warp, by all of its
 // threads.  A kernel that runs beside another one of the wave can start while
 // that one sets the error word; threads that meet at a barrier, a vote or a
-// shared array later must not have read different answers.
+// shared array later must not have read different answers.  Kernels read their
+// queue's length ahead of it, so that the two loads travel together: behind it
+// the viewer frame and the batch were 0.3-0.4% slower.
 __device__ __forceinline__ bool block_failed(const WaveCounters &wc) { return __syncthreads_or(wave_failed(wc)) != 0; }
 __device__ __forceinline__ bool warp_failed(const WaveCounters &wc)
 {

@@ -305,9 +305,9 @@ template <bool COUNT, bool SPLIT, bool BATCH, bool INST = false>
 __global__ void __launch_bounds__(128, INST ? PHC_TRACE_MIN_BLOCKS_INST : PHC_TRACE_MIN_BLOCKS) k_trace(DevScene sc, BatchTable bt, PathSoA in, float4 *__restrict__ hits,
     WaveCounters wc, int it, uint64_t *stats, uint32_t refill, HitQueues hq)
 {
+  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   if (warp_failed(wc))
     return;
-  const uint32_t n = *wc.at(WaveCounters::COUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_TRACE, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
@@ -457,10 +457,10 @@ template <bool BATCH>
 __global__ void __launch_bounds__(256) k_mat_hist(DevScene sc, BatchTable bt, const uint4 *__restrict__ info,
     const float4 *__restrict__ hits, HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
+  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (block_failed(wc))
     return;
   __shared__ uint32_t h[MAT_SORT_BINS];
-  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (n < hq.sort_threshold)
     return;
   for (uint32_t b = threadIdx.x; b < MAT_SORT_BINS; b += blockDim.x)
@@ -477,10 +477,11 @@ __global__ void __launch_bounds__(256) k_mat_hist(DevScene sc, BatchTable bt, co
 // One block of MAT_SORT_BINS threads: bins[0..) counts -> bins[MAT_SORT_BINS..) starts.
 __global__ void __launch_bounds__(MAT_SORT_BINS) k_mat_scan(HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
+  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (block_failed(wc))
     return;
   __shared__ uint32_t t[MAT_SORT_BINS];
-  if (*wc.at(WaveCounters::HCOUNT, it) < hq.sort_threshold)
+  if (n < hq.sort_threshold)
     return;
   const uint32_t b = threadIdx.x;
   t[b] = bins[b];
@@ -502,10 +503,10 @@ template <bool BATCH>
 __global__ void __launch_bounds__(256) k_mat_scatter(DevScene sc, BatchTable bt, const uint4 *__restrict__ info,
     const float4 *__restrict__ hits, HitQueues hq, WaveCounters wc, int it, uint32_t *bins)
 {
+  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (block_failed(wc))
     return;
   __shared__ uint32_t cnt[MAT_SORT_BINS];
-  const uint32_t n = *wc.at(WaveCounters::HCOUNT, it);
   if (n < hq.sort_threshold)
     return;
   uint32_t *start = bins + MAT_SORT_BINS;
@@ -550,9 +551,9 @@ template <bool COUNT, bool BATCH, bool DEFER = false, bool INST = false>
 __global__ void __launch_bounds__(128) k_shadow(const RenderConst *__restrict__ rcp, DevScene sc, BatchTable bt,
     ShadowSoA sh, Accum acc_param, WaveCounters wc, int it, uint64_t *stats, uint32_t refill)
 {
+  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   if (warp_failed(wc))
     return;
-  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_SHADOW, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
@@ -654,13 +655,13 @@ template <bool BATCH>
 __global__ void __launch_bounds__(128) k_shadow_volume(const RenderConst *__restrict__ rcp, DevScene sc,
     BatchTable bt, ShadowSoA sh, Accum acc_param, WaveCounters wc, int it, unsigned long long *lookups)
 {
+  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   if (warp_failed(wc))
     return;
   // the unoccluded shadow rays (tmax >= 0) of the iteration: ratio-tracking
   // transmittance (stream dimension 0x10000 + iteration) times the NEE
   // contribution into the path's pixel slot; persistent warps with refill,
   // one tracking pass per busy lane and trip, as in k_vol_scatter
-  const uint32_t n = *wc.at(WaveCounters::SCOUNT, it);
   uint32_t *fetch = wc.at(WaveCounters::F_VSHADOW, it);
   const uint32_t per_warp = spread_lanes(n);
   // lanes of this warp that take rays
